@@ -5,6 +5,19 @@
 
 #ifdef OWL_EMU
 #include "owl_emu_rt.hpp"
+namespace owl {
+// one host thread per CUDA thread: pollers must leave the cores to the threads that they wait for
+inline void poll_pause() { std::this_thread::sleep_for(std::chrono::milliseconds(20)); }
+inline void warp_sync(unsigned) { emu_t.cta->warpBar[emu_t.tid.x / 32]->arrive_and_wait(); }
+inline void ld_relaxed2(const long long* p, long long& a, long long& b) {
+  a = ld_relaxed(p);
+  b = ld_relaxed(p + 1);
+}
+inline void st_relaxed2(long long* p, long long a, long long b) {
+  st_relaxed(p, a);
+  st_relaxed(p + 1, b);
+}
+}  // namespace owl
 #else
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -14,6 +27,7 @@
 #define OWL_SHARED_ARR(T, name, n) __shared__ T name[n]
 
 namespace owl {
+__device__ __forceinline__ void warp_sync(unsigned mask) { __syncwarp(mask); }
 __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -23,14 +37,18 @@ __device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) {
   asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 // a carry word, read and written by single threads of different CTAs without further ordering: each
-// word carries its own validity (nonzero), so no fence or flag orders it against other data
+// word carries its own validity (its tag), so no fence or flag orders it against other data
 __device__ __forceinline__ long long ld_relaxed(const long long* p) {
   long long v;
   asm volatile("ld.relaxed.gpu.global.s64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_relaxed(long long* p, long long v) {
-  asm volatile("st.relaxed.gpu.global.s64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+// two neighbouring words (16-byte aligned), each of them read or written whole
+__device__ __forceinline__ void ld_relaxed2(const long long* p, long long& a, long long& b) {
+  asm volatile("ld.relaxed.gpu.global.v2.s64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_relaxed2(long long* p, long long a, long long b) {
+  asm volatile("st.relaxed.gpu.global.v2.s64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
 }
 __device__ __forceinline__ unsigned long long gtimer() {
   unsigned long long t;
@@ -40,6 +58,7 @@ __device__ __forceinline__ unsigned long long gtimer() {
 // the carry lookback polls without sleeping: each poll is already an L2 round trip, and a
 // __nanosleep between polls measured 1.4 us slower per line pass at 8M
 __device__ __forceinline__ void spin_pause() {}
+__device__ __forceinline__ void poll_pause() {}
 
 // Programmatic dependent launch. A kernel launched with programmatic stream serialization may be
 // scheduled while the previous kernel on its stream is still finishing: griddep_wait() returns once

@@ -232,50 +232,86 @@ template <int R, int N, int PS, int VPT = 16> __device__ __forceinline__ void st
   }
 }
 
-// tab: this stage's [r][k] table, entry r * NS + k = w_(R NS)^(r k). For
-// radix 8 and 16 only the rows r = 1 and r = 4 are read; the other powers come
-// from at most three products of those two correctly rounded values (each
-// within a few ulp), which keeps the L1 data path free for the exchanges.
+// Stage twiddles. tab is the stage's [r][k] table, entry r * NS + k = w_(R NS)^(r k); the rows r = 1, 2,
+// 4, 8 are read (each correctly rounded) and the other powers are one or two products of them, which
+// keeps the L1 data path free for the exchanges.
+//
+// Twist: the inter-pass twiddle w_hN^(x y) of line x, y the index along it, rides on the stage twiddles
+// of the transform that reads it: a stage of radix R at product NS has the step w_(NS R)^k d with
+// d = w_hN^(x N/(NS R)) instead of w_(NS R)^k, so that the multiplication of every point (8 FP64
+// instructions a point for generating and applying it) becomes one product per table value and, in the
+// first stage, one multiplication. d[e * ds] for e = 0 .. 3 is d, d^2, d^4, d^8 (read if TWIST).
 template <bool INV> __device__ __forceinline__ void twmul(C& v, C w) { v = cmulw<INV>(v, w); }
-
-template <int R, int N, int NS, bool INV, int VPT = 16>
-__device__ __forceinline__ void st_twiddle(int tl, C* v, const C* __restrict__ tab) {
-  if constexpr (NS > 1) {
-#pragma unroll
-    for (int b = 0; b < st_nb<R, VPT>(); ++b) {
-      int j = tl + (N / VPT) * b;
-      if (!st_has<R, N, VPT>(j)) { continue; }
-      int k = smod<NS>(j);
-      C* x = v + b * R;
-      if constexpr (R >= 8) {
-        const C w1 = __ldg(tab + 1 * NS + k);
-        const C w4 = __ldg(tab + 4 * NS + k);
-        const C w2 = csq(w1);
-        const C w3 = cmul(w2, w1);
-        twmul<INV>(x[1], w1);
-        twmul<INV>(x[2], w2);
-        twmul<INV>(x[3], w3);
-        twmul<INV>(x[4], w4);
+template <int R, bool TWIST>
+__device__ __forceinline__ C tw_row(const C* __restrict__ tab, int ns, int k, int e, const C* d, int ds) {
+  C w = __ldg(tab + (1 << e) * ns + k);
+  if constexpr (TWIST) { w = cmul(w, d[e * ds]); }
+  return w;
+}
+template <int R, bool INV, bool TWIST>
+__device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, int k, const C* d = nullptr, int ds = 1) {
+  const C w1 = tw_row<R, TWIST>(tab, ns, k, 0, d, ds);
+  twmul<INV>(x[1], w1);
+  if constexpr (R > 2) {
+    const C w2 = tw_row<R, TWIST>(tab, ns, k, 1, d, ds);
+    const C w3 = (R == 5) ? __ldg(tab + 3 * ns + k) : cmul(w1, w2);
+    twmul<INV>(x[2], w2);
+    twmul<INV>(x[3], w3);
+    if constexpr (R > 4) {
+      const C w4 = tw_row<R, TWIST>(tab, ns, k, 2, d, ds);
+      twmul<INV>(x[4], w4);
+      if constexpr (R > 5) {
         twmul<INV>(x[5], cmul(w4, w1));
         twmul<INV>(x[6], cmul(w4, w2));
         twmul<INV>(x[7], cmul(w4, w3));
-        if constexpr (R == 16) {
-          const C w8 = csq(w4);
-          const C w12 = cmul(w8, w4);
-          twmul<INV>(x[8], w8);
-          twmul<INV>(x[9], cmul(w8, w1));
-          twmul<INV>(x[10], cmul(w8, w2));
-          twmul<INV>(x[11], cmul(w8, w3));
-          twmul<INV>(x[12], w12);
-          twmul<INV>(x[13], cmul(w12, w1));
-          twmul<INV>(x[14], cmul(w12, w2));
-          twmul<INV>(x[15], cmul(w12, w3));
-        }
-      } else {
-#pragma unroll
-        for (int r = 1; r < R; ++r) { twmul<INV>(x[r], __ldg(tab + r * NS + k)); }
+      }
+      if constexpr (R == 16) {
+        const C w8 = tw_row<R, TWIST>(tab, ns, k, 3, d, ds);
+        const C w12 = cmul(w8, w4);
+        twmul<INV>(x[8], w8);
+        twmul<INV>(x[9], cmul(w8, w1));
+        twmul<INV>(x[10], cmul(w8, w2));
+        twmul<INV>(x[11], cmul(w8, w3));
+        twmul<INV>(x[12], w12);
+        twmul<INV>(x[13], cmul(w12, w1));
+        twmul<INV>(x[14], cmul(w12, w2));
+        twmul<INV>(x[15], cmul(w12, w3));
       }
     }
+  }
+}
+
+// the stage twiddles times base (radix 8 and 16; forward)
+template <int R> __device__ __forceinline__ void tw_mul_base(C* x, const C* __restrict__ tab, int ns, int k, C base) {
+  static_assert(R == 8 || R == 16, "radix");
+  const C w1 = __ldg(tab + ns + k), w2 = __ldg(tab + 2 * ns + k), w4 = __ldg(tab + 4 * ns + k);
+  const C lo[4] = {w1, w1, w2, cmul(w1, w2)};
+  C hi[4] = {base, cmul(base, w4), base, base};
+  if constexpr (R == 16) {
+    const C w8 = __ldg(tab + 8 * ns + k);
+    hi[2] = cmul(base, w8);
+    hi[3] = cmul(hi[1], w8);
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) { x[r] = cmul(x[r], (r & 3) == 0 ? hi[r >> 2] : cmul(hi[r >> 2], lo[r & 3])); }
+}
+
+// radix-R butterfly of inputs that carry the stage twiddles
+template <int R, bool INV, bool TWIST>
+__device__ __forceinline__ void tw_dft(C* x, const C* __restrict__ tab, int ns, int k, const C* d, int ds = 1) {
+  static_assert(!TWIST || R != 5, "twisted radix");
+  tw_mul<R, INV, TWIST>(x, tab, ns, k, d, ds);
+  dftR<R, INV>(x);
+}
+
+// twiddles and DFTs of a Stockham stage (NS > 1)
+template <int R, int N, int NS, bool INV, int VPT = 16>
+__device__ __forceinline__ void st_tdft(int tl, C* v, const C* __restrict__ tab) {
+#pragma unroll
+  for (int b = 0; b < st_nb<R, VPT>(); ++b) {
+    int j = tl + (N / VPT) * b;
+    if (!st_has<R, N, VPT>(j)) { continue; }
+    tw_dft<R, INV, false>(v + b * R, tab, NS, smod<NS>(j), nullptr);
   }
 }
 
@@ -301,16 +337,16 @@ template <int R, int N, int NS, int PS, int VPT = 16> __device__ __forceinline__
 // n = 2^a or 5 * 2^a; the factor 5 becomes the M2 stage. r1f != 0 forces the
 // first radix (the split-precision column pass runs a 32-point first stage).
 // vmax: the largest radix (the values per thread).
-constexpr int plan_r1(int n, int rl, int r1f = 0, int vmax = 16) {
+__host__ __device__ constexpr int plan_r1(int n, int rl, int r1f = 0, int vmax = 16) {
   return r1f ? r1f : (n / rl >= vmax ? vmax : n / rl);
 }
-constexpr int plan_rest2(int n, int rl, int r1f = 0, int vmax = 16) { return n / rl / plan_r1(n, rl, r1f, vmax); }
-constexpr int plan_m1(int n, int rl, int r1f = 0, int vmax = 16) {
+__host__ __device__ constexpr int plan_rest2(int n, int rl, int r1f = 0, int vmax = 16) { return n / rl / plan_r1(n, rl, r1f, vmax); }
+__host__ __device__ constexpr int plan_m1(int n, int rl, int r1f = 0, int vmax = 16) {
   return plan_rest2(n, rl, r1f, vmax) % 5 == 0
              ? plan_rest2(n, rl, r1f, vmax) / 5
              : (plan_rest2(n, rl, r1f, vmax) >= vmax ? vmax : plan_rest2(n, rl, r1f, vmax));
 }
-constexpr int plan_m2(int n, int rl, int r1f = 0, int vmax = 16) {
+__host__ __device__ constexpr int plan_m2(int n, int rl, int r1f = 0, int vmax = 16) {
   return plan_rest2(n, rl, r1f, vmax) / plan_m1(n, rl, r1f, vmax);
 }
 
@@ -358,7 +394,24 @@ constexpr TwOffsets tw_offsets(int n, int rl, int r1f = 0, int vmax = 16) {
   return o;
 }
 
+// Whether a pair of n-point rows runs its middle exchanges inside warps (Wl): a power of two whose
+// first radix hands every warp whole sub-transforms. False for the 5 * 2^k columns (16 sub-transforms
+// do not divide among 5 * 2^i warps) and for 2048 points at 8 values a thread (8 sub-transforms, 16 warps).
+__host__ __device__ constexpr bool wl_ok(int n, int rl, int vmax) {
+  return (n & (n - 1)) == 0 && (2 * n / vmax <= 32 || plan_r1(n, rl, 0, vmax) % (2 * n / vmax / 32) == 0);
+}
+// the column t' of thread t in a Wl transform's radix-RL stage, and back
+__host__ __device__ constexpr int wl_col(int n, int rl, int vmax, int t) {
+  const int r1 = plan_r1(n, rl, 0, vmax), m = n / rl / r1;
+  return t / m + r1 * (t % m);
+}
+__host__ __device__ constexpr int wl_thr(int n, int rl, int vmax, int c) {
+  const int r1 = plan_r1(n, rl, 0, vmax), m = n / rl / r1;
+  return (c % r1) * m + c / r1;
+}
+
 template <int N, int RL, int R1F = 0, int VPT = 16> struct Plan {
+  static constexpr int RLAST = RL;
   static constexpr int R1 = plan_r1(N, RL, R1F, VPT);
   static constexpr int M1 = plan_m1(N, RL, R1F, VPT);
   static constexpr int M2 = plan_m2(N, RL, R1F, VPT);
@@ -369,5 +422,142 @@ template <int N, int RL, int R1F = 0, int VPT = 16> struct Plan {
   static_assert(M2 == 5 || (VPT % M2 == 0), "plan: second middle radix 5 or a divisor of the values per thread");
   static_assert(R1 >= 4, "first radix too small for conflict-free padding");
 };
+
+// What the line pass needs to know of a group of two lines x = 2 g, 2 g + 1, one contiguous record that
+// the CTA copies to shared memory while its state loads are under way (entry i of line x at 2 i + x % 2):
+// the first stage's steps w_hN^(x r W/R1), r < 16; the twists d, d^2, d^4, d^8 of the stages M1 and M2
+// and d, d^2, d^4 of the radix-RL stage; w_hN^(x j) as LO[j % 16] HI[j / 16], or for the second of paired
+// lanes w_hN^(x (j - W)) as LO[j % 16] HIB[j / 16]; the lines' weights (wt2 and iwt2 of words e = 0, 1).
+// Read one by one where they are used, every one of these was an L2 round trip of its own per CTA, and
+// the two-level w_hN table two gathers of up to 32 wavefronts.
+struct LineTw {
+  static constexpr int M1 = 16, M2 = 20, RL = 24, LO = 27, HI = 43, HIB = 52, WT = 61, IWT = 62, LEN = 63;
+};
+
+// ---- The transform of two rows (lines or columns) whose middle exchanges stay inside a warp ----
+//
+// A CTA of T = 2 N / VPT threads holds two rows of N = R1 M1 M2 RL points. The first (A order) or
+// last (B order) radix-R1 stage leaves R1 independent sub-transforms of S = N / R1 points per row,
+// sub-transform q in the shared-memory region (row, q); a warp then owns the regions of NSUB = R1 /
+// warps values of q in both rows and runs the remaining stages in them with no barrier but its own.
+// One exchange of the transform is left that needs the whole CTA. The line and column passes had two
+// barriers per exchange, 9 to 11 per launch, now 2: at 8M barriers were the line pass's top stall.
+//
+// Index maps, A order (input index i = j + S r, output index n = q + R1 (p + M n2), M = M1 M2,
+// p = p1 + M1 p2; B order is the same graph backwards):
+//   region (row, q) starts at row RS + q SQ; after the first stage it holds j at j;
+//   after stage M1 it holds (p, jl) at p (RL + 1) + jl (M2 = 1) or (p1, j') at p1 RL M2 + j';
+//   after stage M2 it holds (p, jl) at p (RL + 1) + jl;
+//   the radix-RL stage runs (q, p) of both rows in thread t = q M + p, whose outputs are n = t' + R1 M n2
+//   with t' = wl_col(t) = q + R1 p. Tables that this stage reads are stored in thread order.
+// Every access is free of bank conflicts: 8 neighbouring lanes read or write 8 neighbouring elements,
+// elements RL + 1 apart, or 4 neighbours in each row with RS = 4 mod 8.
+template <int N, int RL, int VPT = 16> struct Wl {
+  using P = Plan<N, RL, 0, VPT>;
+  static constexpr int R1 = P::R1, M1 = P::M1, M2 = P::M2, M = M1 * M2, S = N / P::R1;
+  static constexpr int T = 2 * N / VPT;
+  static constexpr int NW = T > 32 ? T / 32 : 1;
+  static constexpr int LANES = T > 32 ? 32 : T;
+  static constexpr bool ok = wl_ok(N, RL, VPT);
+  static constexpr int NSUB = R1 / NW;
+  static constexpr int SQ = M * (RL + 1);
+  static constexpr int RS = N + N / RL + 4;
+};
+// barrier of a warp (its first T threads in a CTA of T < 32)
+template <int T> __device__ __forceinline__ void wl_sync() { warp_sync(T >= 32 ? 0xffffffffu : ((1u << (T & 31)) - 1u)); }
+
+// row and q of butterfly group gq (2 NSUB groups a warp); MIRROR: row 1 runs R1 - 1 - q
+template <typename G, bool MIRROR> __device__ __forceinline__ void wl_group(int warp, int gq, int& row, int& q) {
+  // RL = 8: q fastest, RL = 4: the row fastest, so that 8 neighbouring lanes never meet in a bank
+  const int ql = (G::P::RLAST == 4) ? gq / 2 : gq % G::NSUB;
+  row = (G::P::RLAST == 4) ? gq % 2 : gq / G::NSUB;
+  q = warp * G::NSUB + ql;
+  if (MIRROR && row == 1) { q = G::R1 - 1 - q; }
+}
+
+// One middle stage of a warp: radix R; ld / st give the element of (butterfly u, input or output r) inside
+// a region, kf the twiddle index; with TWIST d + row is the row's twist, entries two apart (LineTw).
+template <typename G, bool MIRROR, int R, bool INV, bool TWIST, int VPT, typename LD, typename ST, typename KF>
+__device__ __forceinline__ void wl_stage(C* smem, int t, const C* __restrict__ tab, int ns,
+                                         const C* d, LD ld, ST st, KF kf) {
+  constexpr int U = G::S / R;  // butterflies of a region
+  constexpr int NB = VPT / R;
+  const int warp = t / 32, lane = t % 32;
+  C u[VPT];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int f = lane + G::LANES * b;
+    int row, q;
+    wl_group<G, MIRROR>(warp, f / U, row, q);
+    const C* reg = smem + row * G::RS + q * G::SQ;
+#pragma unroll
+    for (int r = 0; r < R; ++r) { u[b * R + r] = reg[ld(f % U, r)]; }
+  }
+  wl_sync<G::T>();
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    const int f = lane + G::LANES * b;
+    int row, q;
+    wl_group<G, MIRROR>(warp, f / U, row, q);
+    tw_dft<R, INV, TWIST>(u + b * R, tab, ns, kf(f % U, q), d + row, 2);
+    C* reg = smem + row * G::RS + q * G::SQ;
+#pragma unroll
+    for (int r = 0; r < R; ++r) { reg[st(f % U, r)] = u[b * R + r]; }
+  }
+  wl_sync<G::T>();
+}
+
+// the middle stages in A order (after the first stage's block exchange, before the radix-RL stage);
+// TWIST: d is the line group's record (LineTw). GAP: the upper half of every region after the block
+// exchange starts GAP elements late (the line pass's paired lanes)
+template <int N, int RL, int VPT, bool MIRROR, bool INV, bool TWIST, int GAP = 0>
+__device__ __forceinline__ void wl_middle_a(C* smem, int t, const C* __restrict__ tw, const C* d) {
+  using G = Wl<N, RL, VPT>;
+  using P = typename G::P;
+  static_assert(GAP == 0 || G::M1 > 1, "the gap lies before a middle stage");
+  if constexpr (G::M1 > 1) {
+    constexpr int U = G::S / G::M1;  // = RL M2
+    wl_stage<G, MIRROR, G::M1, INV, TWIST, VPT>(
+        smem, t, tw + P::TW.aM1, G::R1, d + 2 * LineTw::M1,
+        [](int u, int r) { return u + U * r + (2 * r >= G::M1 ? GAP : 0); },
+        [](int u, int r) { return G::M2 == 1 ? r * (RL + 1) + u : r * U + u; }, [](int, int q) { return q; });
+  }
+  if constexpr (G::M2 > 1) {
+    wl_stage<G, MIRROR, G::M2, INV, TWIST, VPT>(
+        smem, t, tw + P::TW.aM2, G::R1 * G::M1, d + 2 * LineTw::M2,
+        [](int u, int r) { return (u / RL) * (RL * G::M2) + u % RL + RL * r; },
+        [](int u, int r) { return (u / RL + G::M1 * r) * (RL + 1) + u % RL; },
+        [](int u, int q) { return q + G::R1 * (u / RL); });
+  }
+}
+// the middle stages in B order (after the radix-RL stage, before the last stage's block exchange)
+template <int N, int RL, int VPT, bool MIRROR, bool INV, int GAP = 0>
+__device__ __forceinline__ void wl_middle_b(C* smem, int t, const C* __restrict__ tw) {
+  using G = Wl<N, RL, VPT>;
+  using P = typename G::P;
+  static_assert(GAP == 0 || G::M1 > 1, "the gap lies after a middle stage");
+  if constexpr (G::M2 > 1) {
+    wl_stage<G, MIRROR, G::M2, INV, false, VPT>(
+        smem, t, tw + P::TW.bM2, RL, nullptr,
+        [](int u, int r) { return (u / RL + G::M1 * r) * (RL + 1) + u % RL; },
+        [](int u, int r) { return (u / RL) * (RL * G::M2) + u % RL + RL * r; }, [](int u, int) { return u % RL; });
+  }
+  if constexpr (G::M1 > 1) {
+    constexpr int U = G::S / G::M1;
+    wl_stage<G, MIRROR, G::M1, INV, false, VPT>(
+        smem, t, tw + P::TW.bM1, U, nullptr,
+        [](int u, int r) { return G::M2 == 1 ? r * (RL + 1) + u : r * U + u; },
+        [](int u, int r) { return u + U * r + (2 * r >= G::M1 ? GAP : 0); }, [](int u, int) { return u; });
+  }
+}
+// the region element where thread t's radix-RL inputs (A order) or outputs (B order) of a row start
+template <typename G, bool MIRROR> __device__ __forceinline__ int wl_last(int t, int row) {
+  int q = t / G::M, p = t % G::M;
+  if (MIRROR && row == 1) {
+    q = G::R1 - 1 - q;
+    p = G::M - 1 - p;
+  }
+  return row * G::RS + q * G::SQ + p * (G::P::RLAST + 1);
+}
 
 }  // namespace owl

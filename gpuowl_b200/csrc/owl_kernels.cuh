@@ -5,14 +5,14 @@
 // the reference's kAt(), src/Gpu.cpp:40):
 //
 //   pass 2 ("column" pass, k_pass2): for each column pair (k1, W-k1) of the
-//     W x H matrix A[k1][j2]: twiddle by w_hN^(k1 j2), forward length-H DFT,
+//     W x H matrix A[k1][j2]: forward length-H DFT,
 //     real-signal squaring of Z[k] with Z[hN-k] (reference tailSquare /
-//     pairSq, src/cl/tailsquare.cl:35-74), inverse DFT, untwiddle.
-//   pass 1 ("line" pass, k_pass1): for each group of R lines j2: inverse
+//     pairSq, src/cl/tailsquare.cl:35-74), inverse DFT.
+//   pass 1 ("line" pass, k_pass1): for each group of R lines j2: untwiddle, inverse
 //     length-W DFT, inverse weight, round, balanced-digit carry, publish the
 //     line group's carry-out, take the predecessor's carry-in (decoupled
-//     lookback with a bounded wait), weight, forward length-W DFT (reference
-//     carryFused, src/cl/carryfused.cl:21-231).
+//     lookback with a bounded wait), weight, forward length-W DFT, twiddle by
+//     w_hN^(k1 j2) (reference carryFused, src/cl/carryfused.cl:21-231).
 //
 // Layout of F in HBM: tiles of R lines x one column pair. Element (column k1,
 // line j2) lives at (((j2/R) * (W/2) + c) * 2 + s) * R + j2 % R where the pair
@@ -27,7 +27,7 @@
 namespace owl {
 
 struct Ctl {
-  uint32_t ticket;    // line-group ticket for the carry chain (reset by the last taker)
+  uint32_t ticket;    // line-group ticket for the carry chain (reset by the last taker), and kTicketTag
   uint32_t error;     // DEVERR_* bits, sticky until the host clears them
   uint32_t npending;  // carries left over at the end of a thread's word chain (block exit only)
   uint32_t pad[29];
@@ -41,20 +41,22 @@ struct Args {
   // 8M line pass spilled a register and ran 1.8 us slower)
   double scaleLo;      // 2^bitsLo
   double iscaleLo;     // 2^-bitsLo
-  const C* twW;    // stage tables of the width FFT (tw_offsets(W, 16/R) layout)
-  const C* twH;    // stage tables of the height FFT (tw_offsets(H, V / 2, 0, V) layout, V = col_vpt(variant))
-  const C* rootH;  // w_H^i, i < H
+  const C* twW;    // stage tables of the width FFT (tw_offsets(W, 16/R) layout), then the records of the
+                   // line groups (LineTw)
+  const C* twH;    // stage tables of the height FFT (tw_offsets(H, V / 2, 0, V) layout, V = col_vpt(variant)),
+                   // then w_H^k of the threads (col_stage_tables)
+  const C* rootH;  // w_H^i, i < H (the split-precision column pass)
   const C* twLo;   // w_hN^i, i < 2^loShift
   const C* twHi;   // w_hN^(i << loShift)
-  const double* wt1;   // per column j1: 2^(X1/N)
-  const double* iwt1;  // per column j1: 2^(-X1/N)
+  const double* wt1;   // per column j1: 2^(X1/N), column wl_col(t) + (W/RL) r at 2 (t + (W/RL) (r/2)) + r % 2
+  const double* iwt1;  // per column j1: 2^(-X1/N), in the same order
   const uint32_t* x1;  // per column j1: X1 = step*2H*j1 mod N
   const double* wt2;   // per (line j2, e): 2^(X2/N)
   const double* iwt2;  // per (line j2, e): 2^(-X2/N) / (4 hN)
   const uint32_t* x2;  // per (line j2, e): X2 = step*(2 j2 + e) mod N
   const uint2* p1masks; // per (line group g, pass-1 thread t): the big-word and wrap bits of the thread's
-                        // 32 words, bit (r R + ll) 2 + e for column t + (W/RL) r, line g R + ll, word e
-  long long* shuttle;  // carry words, (H/R) x W; 0 = consumed, else the carry encoded (kCarryOffset)
+                        // 32 words, bit (r R + ll) 2 + e for column wl_col(t) + (W/RL) r, line g R + ll, word e
+  long long* shuttle;  // carry words, (H/R) x W in wt1's order: the carry plus an offset, above a tag bit
   long long* pending;  // (word index, carry) pairs, kPendingCap entries
   uint32_t* flags;     // per line group
   Ctl* ctl;
@@ -76,8 +78,8 @@ enum : int { P1_FUSED = 0, P1_IN = 1, P1_OUT = 2 };
 #include "owl_line_tc.cuh"
 namespace owl {
 
-// smem strides: room for the largest padding used (one pad per 2^PS elements,
-// PS >= 2), rounded so that consecutive lines start 4 elements apart mod 8
+// smem strides: room for one pad per RL elements, rounded so that consecutive lines start 4 elements
+// apart mod 8
 template <int W, int R> constexpr int p1_line_stride() {
   constexpr int ps = ilog2(16 / R) < ilog2(Plan<W, 16 / R>::R1) ? ilog2(16 / R) : ilog2(Plan<W, 16 / R>::R1);
   return W + (W >> ps) + 4;
@@ -115,8 +117,12 @@ __device__ __forceinline__ long long sext_low(long long x, uint32_t bits) {
 }
 
 constexpr double RNDVAL = 3.0 * 2251799813685248.0;  // 3 * 2^51
-// offset of an integer carry word in the carry rows (words are never 0: 0 marks a consumed word)
-constexpr long long kCarryOffset = 1ll << 62;
+// Carry words: twice the FP64 carry's bits as carry + RNDVAL (the integer carry of a block exit plus
+// kCarryOffset), plus the launch's tag.
+constexpr long long kCarryOffset = 1ll << 61;
+// bit of the ticket counter that alternates between launches; a launch that finds it clear uses tag 1, so
+// that the words of a fresh plan (all 0) are not yet there
+constexpr uint32_t kTicketTag = 1u << 31;
 
 // launch timestamps for the profiler: slot < 0 turns them off
 __device__ __forceinline__ void ts_begin(const Args& a, int slot) {
@@ -126,18 +132,35 @@ __device__ __forceinline__ void ts_end(const Args& a, int slot) {
   if (slot >= 0 && threadIdx.x == 0) { atomicMax(a.tsEnd + slot, gtimer()); }
 }
 
-// weight line ll of a pass-1 group: digits dgl[r][e] of column j1 = t + (W/RL) r
+// The line pass reads and writes the state in 128-byte lines: two neighbouring columns c, both sides of
+// the pair and both lines. With lanes on consecutive k1 a request would take only one side of each pair,
+// half of every line, which costs twice the L1 wavefronts (of the passes' 16 a value's exchanges take 8
+// per stage boundary, each state access 8 instead of 4). So lane pairs work on the butterflies j and
+// S - j (S = W/R1): at step i the first takes r = i and the second r = R1 - 1 - i, the mirror column. The
+// second keeps its values conjugated: its transform is then the first's, with the same twiddles (p1_pair).
+// Lines of at least 512 points, where a region of shared memory has the 3 elements to spare that keep the
+// two halves of the pairs in different banks.
+constexpr int kPairMinW = 512;
+constexpr int kPairGap = 3;
+
+// flips the sign of the imaginary part where m is the sign bit
+__device__ __forceinline__ C conj_if(C a, long long m) {
+  return mk(a.x, __longlong_as_double(__double_as_longlong(a.y) ^ m));
+}
+
+// weight line ll of a pass-1 group: digits dgl[r][e] of column j1 = c1 + (W/RL) r, c1 = wl_col(t),
 // times 2^(extra/N), halved where the two table exponents wrap past N
 template <int W, int R>
-__device__ __forceinline__ void p1_weight_line(const Args& a, int t, uint32_t g, int ll, const double (&dgl)[16 / R][2],
+__device__ __forceinline__ void p1_weight_line(const Args& a, int t, const C* dG, int ll, const double (&dgl)[16 / R][2],
                                                uint32_t wrapmask, C* v) {
   constexpr int RL = 16 / R;
-  const uint32_t j2 = g * R + ll;
-  const double w20 = __ldg(a.wt2 + 2 * j2), w21 = __ldg(a.wt2 + 2 * j2 + 1);
+  const C w2 = dG[2 * LineTw::WT + ll];
+  const double w20 = w2.x, w21 = w2.y;
+  C w1r;
 #pragma unroll
   for (int r = 0; r < RL; ++r) {
-    const uint32_t j1 = t + (W / RL) * r;
-    const double w1 = __ldg(a.wt1 + j1);
+    if (r % 2 == 0) { w1r = __ldg(reinterpret_cast<const C*>(a.wt1) + t + (W / RL) * (r / 2)); }
+    const double w1 = (r & 1) ? w1r.y : w1r.x;
     double y0 = dgl[r][0] * (w1 * w20);
     double y1 = dgl[r][1] * (w1 * w21);
     if ((wrapmask >> ((r * R + ll) * 2 + 0)) & 1u) { y0 *= 0.5; }
@@ -148,11 +171,12 @@ __device__ __forceinline__ void p1_weight_line(const Args& a, int t, uint32_t g,
 
 // first forward width stage (radix 16/R, NS = 1) of one line, from registers to
 // shared memory
-template <int W, int R> __device__ __forceinline__ void p1_fwd_first(C* ln, int t, C* vl) {
+template <int W, int R> __device__ __forceinline__ void p1_fwd_first(C* smem, int t, int ll, C* vl) {
   constexpr int RL = 16 / R;
   dftR<RL, false>(vl);
+  C* ln = smem + wl_last<Wl<W, RL>, false>(t, ll);
 #pragma unroll
-  for (int r = 0; r < RL; ++r) { ln[pad<ilog2(RL)>(t * RL + r)] = vl[r]; }
+  for (int r = 0; r < RL; ++r) { ln[r] = vl[r]; }
 }
 
 // Pass 1 (the line pass) runs R lines of W points per CTA, R*W/16 threads, 16 values per thread:
@@ -228,7 +252,6 @@ __device__ __forceinline__ C one_mul(C a, C b, C c, C d, C t2) {
 template <int W, int R, int MODE, bool ROE = true, bool SPLIT = false>
 __global__ void __launch_bounds__(R * W / 16, (R * W / 16 == 256) ? 2 : 1)
     k_pass1(Args a, C* __restrict__ F, int32_t* __restrict__ words, int roeSlot, int flags, int tslot) {
-  constexpr bool REGBOUND = false;
   const uint32_t blk = blockIdx.x;
 #include "owl_pass1_body.inc"
 }
@@ -260,7 +283,6 @@ template <int W, int R, int MODE, bool ROE = true>
 __global__ void __launch_bounds__(R * W / 16, occ_blocks(R * W / 16))
     k_pass1_group(const __grid_constant__ GroupArgs ga, int roeSlot, int flags) {
   constexpr bool SPLIT = false;
-  constexpr bool REGBOUND = true;
   const Args& a = ga.a[blockIdx.y];
   C* __restrict__ F = ga.F[blockIdx.y];
   int32_t* __restrict__ words = ga.words[blockIdx.y];

@@ -65,12 +65,13 @@ size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // byte layout of the scratch for one shape; returns the total size
 struct Layout {
-  size_t F, shuttle, pending, flags, ctl, roe, twW, twH, rootH, twLo, twHi, wt1, iwt1, x1, wt2, iwt2, x2, masks, total;
+  size_t F, shuttle, pending, flags, ctl, roe, twW, twH, twLo, twHi, wt1, iwt1, x1, wt2, iwt2, x2, masks, total;
 };
 Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   const uint32_t hN = W * H, G = H / kR;
   const int vH = owl::col_vpt(owl::COL_V16);  // the default column variant's kernels
-  const int twWn = owl::tw_offsets((int)W, 16 / kR).total, twHn = owl::tw_offsets((int)H, vH / 2, 0, vH).total;
+  const int twWn = owl::tw_offsets((int)W, 16 / kR).total + (int)H * owl::LineTw::LEN;
+  const int twHn = owl::tw_offsets((int)H, vH / 2, 0, vH).total + (int)H / (vH / 2);
   Layout L{};
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = up256(o + bytes); return at; };
@@ -82,7 +83,6 @@ Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   L.roe = take(kRoeSlots * sizeof(float));
   L.twW = take(twWn * sizeof(owl::C));
   L.twH = take(twHn * sizeof(owl::C));
-  L.rootH = take(H * sizeof(owl::C));
   L.twLo = take((size_t(1) << loShift) * sizeof(owl::C));
   L.twHi = take((hN >> loShift) * sizeof(owl::C) + sizeof(owl::C));
   L.wt1 = take(W * sizeof(double));
@@ -107,6 +107,7 @@ __device__ owl::C droot(uint32_t n, uint64_t k) {
 __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
   const uint32_t W = a.W, H = a.H, N = a.N;
+  const uint64_t step = N - (a.E % N);
   auto stage = [&](owl::C* tab, uint32_t n, uint32_t rl, uint32_t vmax, uint32_t i) {
     const owl::TwOffsets o = owl::tw_offsets((int)n, (int)rl, 0, (int)vmax);
     const uint32_t r1 = owl::plan_r1(n, rl, 0, vmax), m1 = owl::plan_m1(n, rl, 0, vmax),
@@ -121,23 +122,54 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
     else if (m1 > 1 && (int)i >= o.bM1 && (int)i < o.bR1) { off = o.bM1; R = m1; NS = rl * m2; }
     else { off = o.bR1; R = r1; NS = n / r1; }
     const uint32_t e = i - off, r = e / NS, k = e % NS;
-    tab[i] = droot(R * NS, (uint64_t)r * k);
+    // the radix-rl stage's table is in thread order (all shapes here have warp-local exchanges)
+    const bool last = off == o.aRL && (int)i < o.bM2;
+    tab[i] = droot(R * NS, (uint64_t)r * (last ? (uint32_t)owl::wl_col((int)n, (int)rl, (int)vmax, (int)k) : k));
   };
   const uint32_t vH = (uint32_t)owl::col_vpt(owl::COL_V16);
   for (uint32_t i = tid; i < twWn; i += nth) { stage(const_cast<owl::C*>(a.twW), W, 16 / kR, 16, i); }
+  // the line groups' twist tables (line_tables; W here is below the width from which lanes pair)
+  static_assert(kNoAllocMaxW < (uint32_t)owl::kPairMinW, "no-alloc widths");
+  {
+    const uint32_t r1 = owl::plan_r1(W, 16 / kR), d1 = W / (r1 * owl::plan_m1(W, 16 / kR)),
+                   d2 = d1 / owl::plan_m2(W, 16 / kR), len = owl::LineTw::LEN;
+    for (uint32_t i = tid; i < H * len; i += nth) {
+      const uint32_t x = i / (2 * len) * 2 + i % 2;
+      const int e = (int)(i % (2 * len) / 2);
+      const uint64_t m = e < owl::LineTw::M1 ? (e < (int)r1 ? (uint64_t)e * (W / r1) : 0u)
+                         : e < owl::LineTw::M2 ? (uint64_t)d1 << (e - owl::LineTw::M1)
+                         : e < owl::LineTw::RL ? (uint64_t)d2 << (e - owl::LineTw::M2)
+                         : e < owl::LineTw::LO ? (uint64_t)1 << (e - owl::LineTw::RL)
+                         : e < owl::LineTw::HI ? (uint64_t)(e - owl::LineTw::LO)
+                         : e < owl::LineTw::HIB ? (uint64_t)16 * (e - owl::LineTw::HI)
+                                                : a.hN + (uint64_t)16 * (e - owl::LineTw::HIB) - W;
+      if (e < owl::LineTw::WT) {
+        const_cast<owl::C*>(a.twW)[twWn + i] = droot(a.hN, m * x);
+      } else {
+        const double X0 = (double)((step * (uint64_t)(2 * x)) % N) / N, X1 = (double)((step * (uint64_t)(2 * x + 1)) % N) / N;
+        const_cast<owl::C*>(a.twW)[twWn + i] =
+            e == owl::LineTw::WT ? owl::mk(exp2(X0), exp2(X1))
+                                 : owl::mk(exp2(-X0) / (4.0 * (double)a.hN), exp2(-X1) / (4.0 * (double)a.hN));
+      }
+    }
+  }
   for (uint32_t i = tid; i < twHn; i += nth) { stage(const_cast<owl::C*>(a.twH), H, vH / 2, vH, i); }
-  for (uint32_t i = tid; i < H; i += nth) { const_cast<owl::C*>(a.rootH)[i] = droot(H, i); }
+  for (uint32_t i = tid; i < H / (vH / 2); i += nth) {
+    const_cast<owl::C*>(a.twH)[twHn + i] = droot(H, (uint64_t)owl::wl_col((int)H, (int)vH / 2, (int)vH, (int)i));
+  }
   const uint32_t S = 1u << a.loShift;
   for (uint32_t i = tid; i < S; i += nth) { const_cast<owl::C*>(a.twLo)[i] = droot(a.hN, i); }
   for (uint32_t i = tid; i <= (a.hN >> a.loShift); i += nth) {
     const_cast<owl::C*>(a.twHi)[i] = droot(a.hN, (uint64_t)i << a.loShift);
   }
-  const uint64_t step = N - (a.E % N);
   for (uint32_t j1 = tid; j1 < W; j1 += nth) {
     uint32_t X = (uint32_t)((step * 2 * H * (uint64_t)j1) % N);
     const_cast<uint32_t*>(a.x1)[j1] = X;
-    const_cast<double*>(a.wt1)[j1] = exp2((double)X / N);
-    const_cast<double*>(a.iwt1)[j1] = exp2(-(double)X / N);
+    constexpr uint32_t RL = 16 / kR;
+    const uint32_t r = j1 / (W / RL), th = (uint32_t)owl::wl_thr((int)W, (int)RL, 16, (int)(j1 % (W / RL)));
+    const uint32_t at = 2 * (th + W / RL * (r / 2)) + r % 2;
+    const_cast<double*>(a.wt1)[at] = exp2((double)X / N);
+    const_cast<double*>(a.iwt1)[at] = exp2(-(double)X / N);
   }
   for (uint32_t i = tid; i < 2 * H; i += nth) {
     uint32_t X = (uint32_t)((step * (uint64_t)i) % N);
@@ -153,7 +185,7 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
       const uint32_t g = i / T, th = i % T;
       uint32_t big = 0, wrap = 0;
       for (uint32_t r = 0; r < RL; ++r) {
-        const uint32_t j1 = th + (W / RL) * r;
+        const uint32_t j1 = (uint32_t)owl::wl_col((int)W, (int)RL, 16, (int)th) + (W / RL) * r;
         const uint32_t X1 = (uint32_t)((step * 2 * H * (uint64_t)j1) % N);
         for (uint32_t ll = 0; ll < kR; ++ll) {
           for (uint32_t e = 0; e < 2; ++e) {
@@ -169,7 +201,7 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
     }
   }
   for (uint32_t i = tid; i < H / kR; i += nth) { a.flags[i] = 0; }
-  // carry words: 0 = consumed (a call that stopped on an error may have left some set)
+  // carry words of tag 0, the tag of the launch before the first
   for (uint32_t i = tid; i < (H / kR) * W; i += nth) { a.shuttle[i] = 0; }
   if (tid == 0) {
     a.ctl->ticket = 0;
@@ -273,7 +305,6 @@ extern "C" int owl_square_noalloc(int device, uint32_t E, uint32_t W, uint32_t H
   owl::Args a{};
   a.twW = reinterpret_cast<const owl::C*>(base + L.twW);
   a.twH = reinterpret_cast<const owl::C*>(base + L.twH);
-  a.rootH = reinterpret_cast<const owl::C*>(base + L.rootH);
   a.twLo = reinterpret_cast<const owl::C*>(base + L.twLo);
   a.twHi = reinterpret_cast<const owl::C*>(base + L.twHi);
   a.wt1 = reinterpret_cast<const double*>(base + L.wt1);

@@ -364,8 +364,7 @@ __global__ void __launch_bounds__(H / 8, H == 2048 ? 2 : 1)
   __syncthreads();
   // ---- radix-8 middle stage (NS = R1) ----
   st_load<8, H, PS1>(cbuf, tc, u);
-  st_twiddle<8, H, R1, false>(tc, u, twT + P::TW.aM1);
-  st_dft<8, false>(u);
+  st_tdft<8, H, R1, false>(tc, u, twT + P::TW.aM1);
   __syncthreads();
   st_store<8, H, R1, 4>(cbuf, tc, u);
   __syncthreads();
@@ -378,13 +377,8 @@ __global__ void __launch_bounds__(H / 8, H == 2048 ? 2 : 1)
     u[r] = bufA[pad<4>(t + r * T)];
     u[8 + r] = bufB[pad<4>(jB + r * T)];
   }
-#pragma unroll
-  for (int r = 1; r < 8; ++r) {
-    u[r] = cmul(u[r], __ldg(twT + P::TW.aRL + r * T + t));
-    u[8 + r] = cmul(u[8 + r], __ldg(twT + P::TW.aRL + r * T + jB));
-  }
-  dft8<false>(u);
-  dft8<false>(u + 8);
+  tw_dft<8, false, false>(u, twT + P::TW.aRL, T, t, nullptr);
+  tw_dft<8, false, false>(u + 8, twT + P::TW.aRL, T, jB, nullptr);
   if constexpr (MODE == P2_FWD) {
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -447,8 +441,7 @@ __global__ void __launch_bounds__(H / 8, H == 2048 ? 2 : 1)
     }
     __syncthreads();
     st_load<8, H, 3>(cbuf, tc, u);
-    st_twiddle<8, H, 8, true>(tc, u, twT + P::TW.bM1);
-    st_dft<8, true>(u);
+    st_tdft<8, H, 8, true>(tc, u, twT + P::TW.bM1);
     __syncthreads();
     st_store<8, H, 8, 4>(cbuf, tc, u);
     __syncthreads();

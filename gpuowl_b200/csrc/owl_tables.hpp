@@ -13,9 +13,12 @@
 // angle and rounded once to double (the reference builds its tables in long
 // double too, src/TrigBufCache.cpp:22-120).
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <stdexcept>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
@@ -51,6 +54,31 @@ inline HostC root(uint64_t n, uint64_t k) {
   return HostC{(double)c, (double)-s};
 }
 
+// Many roots of one order: w_n^k as a product of two tabulated factors, taken in long double and rounded
+// once (sine and cosine of every entry would make the line groups' records the longest part of making
+// a plan: 105K roots at 8M words).
+class Roots {
+ public:
+  explicit Roots(uint64_t n) : n_(n) {
+    while ((1ull << (2 * sh_)) < n) { ++sh_; }
+    lo_.resize(1ull << sh_);
+    hi_.resize((n >> sh_) + 1);
+    for (uint64_t i = 0; i < lo_.size(); ++i) { root_ld(n, i, &lo_[i].first, &lo_[i].second); }
+    for (uint64_t i = 0; i < hi_.size(); ++i) { root_ld(n, i << sh_, &hi_[i].first, &hi_[i].second); }
+  }
+  HostC at(uint64_t k) const {
+    k %= n_;
+    if (8 * k % n_ == 0) { return root(n_, k); }  // zeros and equal parts exactly
+    const auto &a = lo_[k & ((1ull << sh_) - 1)], &b = hi_[k >> sh_];
+    return HostC{(double)(a.first * b.first - a.second * b.second), -(double)(a.first * b.second + a.second * b.first)};
+  }
+
+ private:
+  uint64_t n_;
+  int sh_ = 0;
+  std::vector<std::pair<long double, long double>> lo_, hi_;  // cos, sin
+};
+
 inline bool is_pow2(uint32_t x) { return x && !(x & (x - 1)); }
 inline uint32_t log2u(uint32_t x) {
   uint32_t r = 0;
@@ -58,29 +86,38 @@ inline uint32_t log2u(uint32_t x) {
   return r;
 }
 
-// the stage twiddle tables of a length-n line FFT in the tw_offsets(n, rl) layout
-inline std::vector<HostC> stage_tables(uint32_t n, uint32_t rl, uint32_t r1f = 0, uint32_t vmax = 16) {
+// the stage twiddle tables of a length-n line FFT in the tw_offsets(n, rl) layout; thread_order: the
+// radix-rl stage's table of a transform with warp-local exchanges, entry k for k = wl_col(thread)
+inline std::vector<HostC> stage_tables(uint32_t n, uint32_t rl, uint32_t r1f = 0, uint32_t vmax = 16,
+                                       bool thread_order = false) {
   const TwOffsets o = tw_offsets((int)n, (int)rl, (int)r1f, (int)vmax);
   const uint32_t r1 = plan_r1(n, rl, r1f, vmax), m1 = plan_m1(n, rl, r1f, vmax), m2 = plan_m2(n, rl, r1f, vmax);
   std::vector<HostC> t(o.total);
-  auto fill = [&](int off, uint32_t R, uint32_t NS) {
+  auto fill = [&](int off, uint32_t R, uint32_t NS, bool perm = false) {
     for (uint32_t r = 0; r < R; ++r) {
-      for (uint32_t k = 0; k < NS; ++k) { t[off + r * NS + k] = root((uint64_t)R * NS, (uint64_t)r * k); }
+      for (uint32_t k = 0; k < NS; ++k) {
+        const uint32_t kk = perm ? (uint32_t)wl_col((int)n, (int)rl, (int)vmax, (int)k) : k;
+        t[off + r * NS + k] = root((uint64_t)R * NS, (uint64_t)r * kk);
+      }
     }
   };
   if (m1 > 1) { fill(o.aM1, m1, r1); }
   if (m2 > 1) { fill(o.aM2, m2, r1 * m1); }
-  fill(o.aRL, rl, n / rl);
+  fill(o.aRL, rl, n / rl, thread_order);
   if (m2 > 1) { fill(o.bM2, m2, rl); }
   if (m1 > 1) { fill(o.bM1, m1, rl * m2); }
   fill(o.bR1, r1, n / r1);
   return t;
 }
 
-// the column FFT's stage tables for a column variant (its values a thread V: tw_offsets(H, V/2, 0, V))
+// the column FFT's stage tables for a column variant (its values a thread V: tw_offsets(H, V/2, 0, V)),
+// and after them w_H^k, k = wl_col(t) (k = t without warp-local exchanges), for its threads t < H / (V/2)
 inline std::vector<HostC> col_stage_tables(uint32_t H, int variant) {
-  const uint32_t v = (uint32_t)col_vpt(variant);
-  return stage_tables(H, v / 2, 0, v);
+  const uint32_t v = (uint32_t)col_vpt(variant), rl = v / 2;
+  const bool wl = wl_ok((int)H, (int)rl, (int)v);
+  std::vector<HostC> r = stage_tables(H, rl, 0, v, wl);
+  for (uint32_t t = 0; t < H / rl; ++t) { r.push_back(root(H, wl ? (uint32_t)wl_col((int)H, (int)rl, (int)v, (int)t) : t)); }
+  return r;
 }
 
 // The column variant a plan of shape W x H starts with: the fastest of the variants built for H as
@@ -93,6 +130,51 @@ inline int default_col_variant(uint32_t W, uint32_t H) {
   if ((W == 128 && H == 256) || (W == 256 && H == 256) || (W == 512 && H == 512)) { return COL_V8; }
   if (W == 4096 && H == 2560) { return COL_V16_OCC2; }
   return COL_V16;
+}
+
+// Whether the line pass pairs its lanes (kPairMinW of the kernels); its inverse transform's first middle
+// stage then reads the half-way row r = M1/2 with the factor that the mirrored butterflies leave on the
+// upper half of their sub-transform, conj(w_2R1^k) for w_2R1^k (and the twist's entry for the same row).
+inline bool line_pairs(uint32_t W) { return W >= 512; }
+
+// the line pass's tables: the stage tables of W points, then the record of every line group (LineTw);
+// wt2 and iwt2: the weights of the words of every line
+inline std::vector<HostC> line_tables(uint32_t W, uint32_t H, const double* wt2, const double* iwt2) {
+  const uint32_t rl = 8;
+  const uint64_t hN = (uint64_t)W * H;
+  const Roots roots(hN);
+  std::vector<HostC> t = stage_tables(W, rl, 0, 16, true);
+  const TwOffsets o = tw_offsets((int)W, (int)rl);
+  const uint32_t r1 = plan_r1(W, rl), m1 = plan_m1(W, rl), m2 = plan_m2(W, rl);
+  const bool pairs = line_pairs(W);
+  if (pairs) {
+    for (uint32_t k = 0; k < r1; ++k) {
+      HostC& w = t[o.aM1 + m1 / 2 * r1 + k];
+      w.y = -w.y;
+    }
+  }
+  const size_t at = t.size();
+  t.resize(at + (size_t)H * LineTw::LEN);
+  for (uint32_t x = 0; x < H; ++x) {
+    HostC* e = t.data() + at + (size_t)(x / 2) * (2 * LineTw::LEN) + x % 2;
+    auto put = [&](int i, uint64_t m) { e[2 * i] = roots.at(m * x); };
+    for (uint32_t r = 0; r < 16; ++r) { put((int)r, r < r1 ? r * (W / r1) : 0); }
+    const uint32_t d1 = W / (r1 * m1), d2 = d1 / m2;
+    for (int i = 0; i < 4; ++i) {
+      put(LineTw::M1 + i, (uint64_t)d1 << i);
+      put(LineTw::M2 + i, (uint64_t)d2 << i);
+      if (i < 3) { put(LineTw::RL + i, 1u << i); }
+      if (pairs && (2u << i) == m1) { put(LineTw::M1 + i, W / 32 * 31); }
+    }
+    for (uint32_t j = 0; j < 16; ++j) { put(LineTw::LO + (int)j, j); }
+    for (uint32_t j = 0; j < (pairs ? 9u : 1u); ++j) {
+      put(LineTw::HI + (int)j, 16 * j);
+      put(LineTw::HIB + (int)j, hN + 16 * j - W);  // mod hN
+    }
+    e[2 * LineTw::WT] = HostC{wt2[2 * x], wt2[2 * x + 1]};
+    e[2 * LineTw::IWT] = HostC{iwt2[2 * x], iwt2[2 * x + 1]};
+  }
+  return t;
 }
 
 struct Tables {
@@ -142,32 +224,49 @@ inline bool shape_for(uint32_t n, uint32_t* W, uint32_t* H) {
 }
 
 // The big-word and wrap bits of every pass-1 thread's words: thread t of line group g holds
-// column j1 = t + (W/RL) r (r < RL = 16/R) of lines j2 = g R + ll (ll < R), words e = 0, 1;
+// column j1 = wl_col(t) + (W/RL) r (r < RL = 16/R) of lines j2 = g R + ll (ll < R), words e = 0, 1;
 // bit (r R + ll) 2 + e. With X = X1[j1] + X2[2 j2 + e], the weight wraps when X >= N and the
 // word is big when X mod N < E mod N.
 inline std::vector<uint32_t> word_masks(uint32_t E, uint32_t W, uint32_t H, const uint32_t* x1, const uint32_t* x2) {
-  const uint32_t R = kLinesPerBlock, RL = 16 / R, T = R * W / 16, G = H / R, N = 2 * W * H;
-  std::vector<uint32_t> m(2 * (size_t)G * T);
-  for (uint32_t g = 0; g < G; ++g) {
-    for (uint32_t th = 0; th < T; ++th) {
-      uint32_t big = 0, wrap = 0;
-      for (uint32_t r = 0; r < RL; ++r) {
-        const uint32_t j1 = th + (W / RL) * r;
-        for (uint32_t ll = 0; ll < R; ++ll) {
-          const uint32_t j2 = g * R + ll;
-          for (uint32_t e = 0; e < 2; ++e) {
-            const uint32_t bit = (r * R + ll) * 2 + e;
-            const uint32_t X = x1[j1] + x2[2 * j2 + e];
-            const bool w = X >= N;
-            if (w) { wrap |= 1u << bit; }
-            if ((w ? X - N : X) < E % N) { big |= 1u << bit; }
+  constexpr uint32_t R = kLinesPerBlock, RL = 16 / R;
+  const uint32_t T = R * W / 16, G = H / R, N = 2 * W * H, em = E % N;
+  std::vector<uint32_t> m(2 * (size_t)G * T), xt(W);  // xt: X1 in thread order
+  for (uint32_t th = 0; th < T; ++th) {
+    const uint32_t c = (uint32_t)wl_col((int)W, (int)RL, 16, (int)th);
+    for (uint32_t r = 0; r < RL; ++r) { xt[th * RL + r] = x1[c + (W / RL) * r]; }
+  }
+  auto groups = [&](uint32_t g0, uint32_t g1) {
+    for (uint32_t g = g0; g < g1; ++g) {
+      uint32_t xl[2 * R];
+      for (uint32_t i = 0; i < 2 * R; ++i) { xl[i] = x2[2 * R * g + i]; }
+      for (uint32_t th = 0; th < T; ++th) {
+        uint32_t big = 0, wrap = 0;
+        for (uint32_t r = 0; r < RL; ++r) {
+          for (uint32_t i = 0; i < 2 * R; ++i) {  // i = 2 ll + e
+            const uint32_t X = xt[th * RL + r] + xl[i], w = X >= N;
+            wrap |= w << (r * 2 * R + i);
+            big |= (uint32_t)(X - (N & (0u - w)) < em) << (r * 2 * R + i);
           }
         }
+        m[2 * ((size_t)g * T + th)] = big;
+        m[2 * ((size_t)g * T + th) + 1] = wrap;
       }
-      m[2 * ((size_t)g * T + th)] = big;
-      m[2 * ((size_t)g * T + th) + 1] = wrap;
+    }
+  };
+  // 2 ns a word: 40 ms at 20M words on one thread
+  const unsigned nt = N < (1u << 20) ? 1u : std::max(1u, std::min(std::thread::hardware_concurrency(), 8u));
+  std::vector<std::thread> pool;
+  pool.reserve(nt);
+  for (unsigned i = 1; i < nt; ++i) {
+    const uint32_t g0 = (uint32_t)((uint64_t)G * i / nt), g1 = (uint32_t)((uint64_t)G * (i + 1) / nt);
+    try {
+      pool.emplace_back(groups, g0, g1);
+    } catch (const std::system_error&) {
+      groups(g0, g1);
     }
   }
+  groups(0, (uint32_t)((uint64_t)G / nt));
+  for (auto& x : pool) { x.join(); }
   return m;
 }
 
@@ -181,7 +280,6 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
   t.N = 2 * W * H;
   const uint32_t N = t.N;
   t.loShift = (log2u(t.hN) + 1) / 2;
-  t.twW = stage_tables(W, 16 / kLinesPerBlock);
   t.twH = col_stage_tables(H, COL_V16);
   t.rootH.resize(H);
   for (uint32_t i = 0; i < H; ++i) { t.rootH[i] = root(H, i); }
@@ -199,8 +297,12 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
   for (uint32_t j1 = 0; j1 < W; ++j1) {
     uint32_t X = (uint32_t)((step * 2 * H * (uint64_t)j1) % N);
     t.x1[j1] = X;
-    t.wt1[j1] = (double)exp2l((long double)X / N);
-    t.iwt1[j1] = (double)exp2l(-(long double)X / N);
+    // in the line pass's thread order
+    constexpr uint32_t RL = 16 / kLinesPerBlock;
+    const uint32_t r = j1 / (W / RL), th = (uint32_t)wl_thr((int)W, (int)RL, 16, (int)(j1 % (W / RL)));
+    const uint32_t at = 2 * (th + W / RL * (r / 2)) + r % 2;
+    t.wt1[at] = (double)exp2l((long double)X / N);
+    t.iwt1[at] = (double)exp2l(-(long double)X / N);
   }
   t.x2.resize(2 * H);
   t.wt2.resize(2 * H);
@@ -212,6 +314,7 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
     t.wt2[i] = (double)exp2l((long double)X / N);
     t.iwt2[i] = (double)(exp2l(-(long double)X / N) * norm);
   }
+  t.twW = line_tables(W, H, t.wt2.data(), t.iwt2.data());
   t.p1masks = word_masks(E, W, H, t.x1.data(), t.x2.data());
   return t;
 }

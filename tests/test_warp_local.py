@@ -1,0 +1,39 @@
+"""The passes whose exchanges stay inside warps, at the widths and heights where their geometry changes:
+CTAs below a warp, of one warp and of several, with and without paired lanes, with one and two middle
+stages. Results are whole numbers and must equal GMP's."""
+import numpy as np
+import pytest
+
+from conftest import random_words
+from test_emulator import emu, run  # noqa: F401  (emu is a fixture)
+
+EDGES = [(64, 64), (128, 64), (256, 64), (512, 64), (1024, 64), (2048, 64), (4096, 64),
+         (64, 128), (64, 256), (64, 512), (64, 1024), (64, 2048), (64, 4096), (64, 640), (64, 1280), (64, 2560)]
+
+
+def exponent(W, H, bpw=16.3):
+    return int(2 * W * H * bpw) | 1
+
+
+@pytest.mark.parametrize("W,H,n,flags", [(256, 64, 3, 0), (512, 64, 3, 2), (64, 512, 2, 0)])
+def test_emulated_edges(emu, oracle, W, H, n, flags):  # noqa: F811
+    E = exponent(W, H)
+    _, got = run(emu, "square", E, W, H, n, flags, 9)
+    assert np.array_equal(got, oracle.gmp_square(E, random_words(E, 9), n, ll=bool(flags & 2)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", EDGES)
+def test_edges_vs_gmp(oracle, W, H):
+    import gpuowl_b200 as owl
+    E = exponent(W, H)
+    wa, wb = random_words(E, 21), random_words(E, 22)
+    with owl.Plan(E, W=W, H=H) as p:
+        a, b = p.alloc(), p.alloc()
+        p.writeIn(a, wa)
+        p.writeIn(b, wb)
+        p.squareLoop(a, a, 18, roe=False)  # a graph: the tags of the carry words alternate
+        p.squareLoop(a, a, 3, ll=True)
+        p.modMul(a, b)
+        want = oracle.gmp_square(E, oracle.gmp_square(E, wa, 18), 3, ll=True)
+        assert np.array_equal(p.readOut(a), oracle.gmp_mul(E, want, wb))
