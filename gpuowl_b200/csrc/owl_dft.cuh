@@ -24,6 +24,10 @@ __device__ __forceinline__ C cmul(C a, C b) {
 __device__ __forceinline__ C cmulc(C a, C b) {
   return mk(fma(a.x, b.x, a.y * b.y), fma(a.y, b.x, -a.x * b.y));
 }
+// a + b c in four FMAs
+__device__ __forceinline__ C caddmul(C a, C b, C c) {
+  return mk(fma(b.x, c.x, fma(-b.y, c.y, a.x)), fma(b.x, c.y, fma(b.y, c.x, a.y)));
+}
 __device__ __forceinline__ C csq(C a) { return mk(fma(a.x, a.x, -a.y * a.y), 2.0 * a.x * a.y); }
 // multiply by i
 __device__ __forceinline__ C cmuli(C a) { return mk(-a.y, a.x); }
@@ -112,26 +116,33 @@ template <bool INV> __device__ __forceinline__ void dft4s(C& x0, C& x1, C& x2, C
 
 template <bool INV> __device__ __forceinline__ void dft4(C* v) { dft4s<INV>(v[0], v[1], v[2], v[3]); }
 
-// 8 = 4 (over n1, stride 2) x 2
+// t with w8 a = kSQ t: a factor w8 costs two additions, and the kSQ rides on the FMAs that take the product
+template <bool INV> __device__ __forceinline__ C w8_sum(C a) {
+  return INV ? mk(a.x - a.y, a.x + a.y) : mk(a.x + a.y, a.y - a.x);
+}
+// a +- kSQ t
+__device__ __forceinline__ C addq(C a, C t) { return mk(fma(kSQ, t.x, a.x), fma(kSQ, t.y, a.y)); }
+__device__ __forceinline__ C subq(C a, C t) { return mk(fma(-kSQ, t.x, a.x), fma(-kSQ, t.y, a.y)); }
+
+// 8 = 4 (over n1, stride 2) x 2: 52 FP64 instructions (56 with the factors w8, w8^3 multiplied out)
 template <bool INV> __device__ __forceinline__ void dft8(C* v) {
   C y0 = v[0], y2 = v[2], y4 = v[4], y6 = v[6];
   C y1 = v[1], y3 = v[3], y5 = v[5], y7 = v[7];
   dft4s<INV>(y0, y2, y4, y6);  // Y0[k1], k1 = 0..3 in (y0, y2, y4, y6)
   dft4s<INV>(y1, y3, y5, y7);  // Y1[k1]
-  y3 = mul_w16<INV, 2>(y3);
-  y5 = mul_w16<INV, 4>(y5);
-  y7 = mul_w16<INV, 6>(y7);
+  const C t3 = w8_sum<INV>(y3), t7 = w8_sum<INV>(mul_w4<INV>(y7));
+  y5 = mul_w4<INV>(y5);
   v[0] = cadd(y0, y1);
   v[4] = csub(y0, y1);
-  v[1] = cadd(y2, y3);
-  v[5] = csub(y2, y3);
+  v[1] = addq(y2, t3);
+  v[5] = subq(y2, t3);
   v[2] = cadd(y4, y5);
   v[6] = csub(y4, y5);
-  v[3] = cadd(y6, y7);
-  v[7] = csub(y6, y7);
+  v[3] = addq(y6, t7);
+  v[7] = subq(y6, t7);
 }
 
-// 16 = 4 (over n1, stride 4) x 4
+// 16 = 4 (over n1, stride 4) x 4: 152 FP64 instructions (160 with the factors w8 multiplied out)
 template <bool INV> __device__ __forceinline__ void dft16(C* v) {
   C y[16];
 #pragma unroll
@@ -139,25 +150,33 @@ template <bool INV> __device__ __forceinline__ void dft16(C* v) {
   // step 1: for n2: DFT4 over n1 of x[4 n1 + n2]; result k1 kept at index n2 + 4 k1
 #pragma unroll
   for (int n2 = 0; n2 < 4; ++n2) { dft4s<INV>(y[n2], y[n2 + 4], y[n2 + 8], y[n2 + 12]); }
-  // step 2: twiddle w16^(n2 k1)
-  y[1 + 4 * 1] = mul_w16<INV, 1>(y[1 + 4 * 1]);
-  y[1 + 4 * 2] = mul_w16<INV, 2>(y[1 + 4 * 2]);
-  y[1 + 4 * 3] = mul_w16<INV, 3>(y[1 + 4 * 3]);
-  y[2 + 4 * 1] = mul_w16<INV, 2>(y[2 + 4 * 1]);
-  y[2 + 4 * 2] = mul_w16<INV, 4>(y[2 + 4 * 2]);
-  y[2 + 4 * 3] = mul_w16<INV, 6>(y[2 + 4 * 3]);
-  y[3 + 4 * 1] = mul_w16<INV, 3>(y[3 + 4 * 1]);
-  y[3 + 4 * 2] = mul_w16<INV, 6>(y[3 + 4 * 2]);
-  y[3 + 4 * 3] = mul_w16<INV, 9>(y[3 + 4 * 3]);
-  // step 3: for k1: DFT4 over n2 -> X[k1 + 4 k2]
-#pragma unroll
-  for (int k1 = 0; k1 < 4; ++k1) {
-    C a = y[0 + 4 * k1], b = y[1 + 4 * k1], c = y[2 + 4 * k1], d = y[3 + 4 * k1];
+  // step 2: for k1: DFT4 over n2 of the values times w16^(n2 k1) -> X[k1 + 4 k2]
+  {
+    C a = y[0], b = y[1], c = y[2], d = y[3];
     dft4s<INV>(a, b, c, d);
-    v[k1 + 0] = a;
-    v[k1 + 4] = b;
-    v[k1 + 8] = c;
-    v[k1 + 12] = d;
+    v[0] = a;
+    v[4] = b;
+    v[8] = c;
+    v[12] = d;
+  }
+#pragma unroll
+  for (int k1 = 1; k1 < 4; k1 += 2) {  // the middle factor is w8 or w8^3
+    const C a = y[4 * k1], t = w8_sum<INV>(k1 == 1 ? y[4 * k1 + 2] : mul_w4<INV>(y[4 * k1 + 2]));
+    const C b = k1 == 1 ? mul_w16<INV, 1>(y[4 * k1 + 1]) : mul_w16<INV, 3>(y[4 * k1 + 1]);
+    const C d = k1 == 1 ? mul_w16<INV, 3>(y[4 * k1 + 3]) : mul_w16<INV, 9>(y[4 * k1 + 3]);
+    const C p = addq(a, t), m = subq(a, t), e = cadd(b, d), f = mul_w4<INV>(csub(b, d));
+    v[k1] = cadd(p, e);
+    v[k1 + 8] = csub(p, e);
+    v[k1 + 4] = cadd(m, f);
+    v[k1 + 12] = csub(m, f);
+  }
+  {  // k1 = 2: the factors w8, w4, w8^3
+    const C a = y[8], c = mul_w4<INV>(y[10]), tb = w8_sum<INV>(y[9]), td = w8_sum<INV>(mul_w4<INV>(y[11]));
+    const C p = cadd(a, c), m = csub(a, c), e = cadd(tb, td), f = mul_w4<INV>(csub(tb, td));
+    v[2] = addq(p, e);
+    v[10] = subq(p, e);
+    v[6] = addq(m, f);
+    v[14] = subq(m, f);
   }
 }
 
@@ -232,9 +251,9 @@ template <int R, int N, int PS, int VPT = 16> __device__ __forceinline__ void st
   }
 }
 
-// Stage twiddles. tab is the stage's [r][k] table, entry r * NS + k = w_(R NS)^(r k); the rows r = 1, 2,
-// 4, 8 are read (each correctly rounded) and the other powers are one or two products of them, which
-// keeps the L1 data path free for the exchanges.
+// Stage twiddles. tab is the stage's [r][k] table, entry r * NS + k = w_(R NS)^(r k); the rows r = 1, 2, 3,
+// 4, 8, 12 are read (each correctly rounded) and the other powers are products of two of them, which
+// keeps the L1 data path free for the exchanges (all rows read: 101.4 us per iteration at 8M, these 100.4).
 //
 // Twist: the inter-pass twiddle w_hN^(x y) of line x, y the index along it, rides on the stage twiddles
 // of the transform that reads it: a stage of radix R at product NS has the step w_(NS R)^k d with
@@ -254,7 +273,7 @@ __device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, 
   twmul<INV>(x[1], w1);
   if constexpr (R > 2) {
     const C w2 = tw_row<R, TWIST>(tab, ns, k, 1, d, ds);
-    const C w3 = (R == 5) ? __ldg(tab + 3 * ns + k) : cmul(w1, w2);
+    const C w3 = TWIST ? cmul(w1, w2) : __ldg(tab + 3 * ns + k);
     twmul<INV>(x[2], w2);
     twmul<INV>(x[3], w3);
     if constexpr (R > 4) {
@@ -267,7 +286,7 @@ __device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, 
       }
       if constexpr (R == 16) {
         const C w8 = tw_row<R, TWIST>(tab, ns, k, 3, d, ds);
-        const C w12 = cmul(w8, w4);
+        const C w12 = TWIST ? cmul(w8, w4) : __ldg(tab + 12 * ns + k);
         twmul<INV>(x[8], w8);
         twmul<INV>(x[9], cmul(w8, w1));
         twmul<INV>(x[10], cmul(w8, w2));
@@ -285,12 +304,12 @@ __device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, 
 template <int R> __device__ __forceinline__ void tw_mul_base(C* x, const C* __restrict__ tab, int ns, int k, C base) {
   static_assert(R == 8 || R == 16, "radix");
   const C w1 = __ldg(tab + ns + k), w2 = __ldg(tab + 2 * ns + k), w4 = __ldg(tab + 4 * ns + k);
-  const C lo[4] = {w1, w1, w2, cmul(w1, w2)};
+  const C lo[4] = {w1, w1, w2, __ldg(tab + 3 * ns + k)};
   C hi[4] = {base, cmul(base, w4), base, base};
   if constexpr (R == 16) {
     const C w8 = __ldg(tab + 8 * ns + k);
     hi[2] = cmul(base, w8);
-    hi[3] = cmul(hi[1], w8);
+    hi[3] = cmul(base, __ldg(tab + 12 * ns + k));
   }
 #pragma unroll
   for (int r = 0; r < R; ++r) { x[r] = cmul(x[r], (r & 3) == 0 ? hi[r >> 2] : cmul(hi[r >> 2], lo[r & 3])); }

@@ -196,11 +196,10 @@ __device__ __forceinline__ void pair_sq(C& a, C& b, C t2) {
   C bc = cconj(b);
   C e2 = cadd(a, bc);
   C o2 = cmulmi(csub(a, bc));
-  C s = cadd(csq(e2), cmul(t2, csq(o2)));
+  C s = caddmul(csq(e2), t2, csq(o2));
   C p = cmuli(cmul(e2, o2));
-  p = mk(2.0 * p.x, 2.0 * p.y);
-  a = cadd(s, p);
-  b = cconj(csub(s, p));
+  a = mk(fma(2.0, p.x, s.x), fma(2.0, p.y, s.y));
+  b = mk(fma(-2.0, p.x, s.x), fma(2.0, p.y, -s.y));
 }
 
 // product of two signals: (a, b) pair of the first, (c, d) of the second
@@ -208,7 +207,7 @@ __device__ __forceinline__ void pair_mul(C& a, C& b, C c, C d, C t2) {
   C bc = cconj(b), dc = cconj(d);
   C e2a = cadd(a, bc), o2a = cmulmi(csub(a, bc));
   C e2b = cadd(c, dc), o2b = cmulmi(csub(c, dc));
-  C s = cadd(cmul(e2a, e2b), cmul(t2, cmul(o2a, o2b)));
+  C s = caddmul(cmul(e2a, e2b), t2, cmul(o2a, o2b));
   C p = cmuli(cadd(cmul(e2a, o2b), cmul(o2a, e2b)));
   a = cadd(s, p);
   b = cconj(csub(s, p));
@@ -219,7 +218,7 @@ __device__ __forceinline__ C one_sq(C a, C b, C t2) {
   C bc = cconj(b);
   C e2 = cadd(a, bc);
   C o2 = cmulmi(csub(a, bc));
-  C s = cadd(csq(e2), cmul(t2, csq(o2)));
+  C s = caddmul(csq(e2), t2, csq(o2));
   C p = cmuli(cmul(e2, o2));
   return cadd(s, mk(2.0 * p.x, 2.0 * p.y));
 }
@@ -227,7 +226,7 @@ __device__ __forceinline__ C one_mul(C a, C b, C c, C d, C t2) {
   C bc = cconj(b), dc = cconj(d);
   C e2a = cadd(a, bc), o2a = cmulmi(csub(a, bc));
   C e2b = cadd(c, dc), o2b = cmulmi(csub(c, dc));
-  C s = cadd(cmul(e2a, e2b), cmul(t2, cmul(o2a, o2b)));
+  C s = caddmul(cmul(e2a, e2b), t2, cmul(o2a, o2b));
   C p = cmuli(cadd(cmul(e2a, o2b), cmul(o2a, e2b)));
   return cadd(s, p);
 }
