@@ -205,8 +205,28 @@ template <bool INV> __device__ __forceinline__ void dft5(C* v) {
   v[3] = cadd(a2, ib2);
 }
 
+// 20 = 4 x 5, coprime factors: n = 5 n1 + 4 n2, k = 5 k1 + 16 k2 (mod 20), no twiddles between
+template <bool INV> __device__ __forceinline__ void dft20(C* v) {
+#pragma unroll
+  for (int n2 = 0; n2 < 5; ++n2) { dft4s<INV>(v[4 * n2], v[(4 * n2 + 5) % 20], v[(4 * n2 + 10) % 20], v[(4 * n2 + 15) % 20]); }
+  C y[20];
+#pragma unroll
+  for (int k1 = 0; k1 < 4; ++k1) {
+    C z[5];
+#pragma unroll
+    for (int n2 = 0; n2 < 5; ++n2) { z[n2] = v[(5 * k1 + 4 * n2) % 20]; }
+    dft5<INV>(z);
+#pragma unroll
+    for (int k2 = 0; k2 < 5; ++k2) { y[(5 * k1 + 16 * k2) % 20] = z[k2]; }
+  }
+#pragma unroll
+  for (int k = 0; k < 20; ++k) { v[k] = y[k]; }
+}
+
 template <int R, bool INV> __device__ __forceinline__ void dftR(C* v) {
-  if constexpr (R == 5) {
+  if constexpr (R == 20) {
+    dft20<INV>(v);
+  } else if constexpr (R == 5) {
     dft5<INV>(v);
   } else if constexpr (R == 2) {
     dft2<INV>(v);
@@ -284,7 +304,7 @@ __device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, 
         twmul<INV>(x[6], cmul(w4, w2));
         twmul<INV>(x[7], cmul(w4, w3));
       }
-      if constexpr (R == 16) {
+      if constexpr (R >= 16) {
         const C w8 = tw_row<R, TWIST>(tab, ns, k, 3, d, ds);
         const C w12 = TWIST ? cmul(w8, w4) : __ldg(tab + 12 * ns + k);
         twmul<INV>(x[8], w8);
@@ -295,6 +315,13 @@ __device__ __forceinline__ void tw_mul(C* x, const C* __restrict__ tab, int ns, 
         twmul<INV>(x[13], cmul(w12, w1));
         twmul<INV>(x[14], cmul(w12, w2));
         twmul<INV>(x[15], cmul(w12, w3));
+        if constexpr (R == 20) {
+          const C w16 = __ldg(tab + 16 * ns + k);
+          twmul<INV>(x[16], w16);
+          twmul<INV>(x[17], cmul(w16, w1));
+          twmul<INV>(x[18], cmul(w16, w2));
+          twmul<INV>(x[19], cmul(w16, w3));
+        }
       }
     }
   }
@@ -355,9 +382,11 @@ template <int R, int N, int NS, int PS, int VPT = 16> __device__ __forceinline__
 // "A order" runs the stages R1, M1, M2, RL; "B order" runs RL, M2, M1, R1.
 // n = 2^a or 5 * 2^a; the factor 5 becomes the M2 stage. r1f != 0 forces the
 // first radix (the split-precision column pass runs a 32-point first stage).
-// vmax: the largest radix (the values per thread).
+// vmax: the largest radix (the values per thread). 2560 and 1280 points at 16 values a thread start with
+// radix 20, run by 4 of every 5 threads: one stage and exchange less than 16 x 4 x 5 x 8, and 20
+// sub-transforms that divide among the CTA's 10 or 5 warps (20M: column pass 169 -> 114 us; 5M: 33 -> 24).
 __host__ __device__ constexpr int plan_r1(int n, int rl, int r1f = 0, int vmax = 16) {
-  return r1f ? r1f : (n / rl >= vmax ? vmax : n / rl);
+  return r1f ? r1f : ((n == 2560 || n == 1280) && rl == 8 && vmax == 16 ? 20 : (n / rl >= vmax ? vmax : n / rl));
 }
 __host__ __device__ constexpr int plan_rest2(int n, int rl, int r1f = 0, int vmax = 16) { return n / rl / plan_r1(n, rl, r1f, vmax); }
 __host__ __device__ constexpr int plan_m1(int n, int rl, int r1f = 0, int vmax = 16) {
@@ -413,11 +442,12 @@ constexpr TwOffsets tw_offsets(int n, int rl, int r1f = 0, int vmax = 16) {
   return o;
 }
 
-// Whether a pair of n-point rows runs its middle exchanges inside warps (Wl): a power of two whose
-// first radix hands every warp whole sub-transforms. False for the 5 * 2^k columns (16 sub-transforms
-// do not divide among 5 * 2^i warps) and for 2048 points at 8 values a thread (8 sub-transforms, 16 warps).
+// Whether a pair of n-point rows runs its middle exchanges inside warps (Wl): its first radix hands every
+// warp whole sub-transforms and leaves a power of two. False for 640 points and for 1280 at 8 values a
+// thread (a factor 5 stays in the middle stages) and for 2048 points at 8 values a thread (8
+// sub-transforms, 16 warps).
 __host__ __device__ constexpr bool wl_ok(int n, int rl, int vmax) {
-  return (n & (n - 1)) == 0 && (2 * n / vmax <= 32 || plan_r1(n, rl, 0, vmax) % (2 * n / vmax / 32) == 0);
+  return plan_rest2(n, rl, 0, vmax) % 5 != 0 && (2 * n / vmax <= 32 || plan_r1(n, rl, 0, vmax) % (2 * n / vmax / 32) == 0);
 }
 // the column t' of thread t in a Wl transform's radix-RL stage, and back
 __host__ __device__ constexpr int wl_col(int n, int rl, int vmax, int t) {
