@@ -243,13 +243,21 @@ __device__ __forceinline__ C one_mul(C a, C b, C c, C d, C t2) {
 // shape in one launch (blockIdx.y = plan), which a batch of exponents uses so that one launch per
 // pass and shape replaces a launch per plan.
 
+// CTAs per SM of the one-plan line pass: 16 warps at 128 registers from 64 threads a CTA (W = 512) up. Free
+// of the bound the 64- and 128-thread kernels took 240-255 registers, 8 warps an SM, which their grids
+// (256 to 1,280 CTAs) more than fill: 4M words 57.1 -> 50.2 us per iteration alone and 53.0 -> 43.8 with
+// three plans in turn, 1M 12.1 -> 9.9 with three plans (alone 17.2 -> 18.6, the one loss: its CTAs then
+// start on fewer SMs). 20 warps (102 registers) spill: 4M 46.0. The narrower kernels run a fraction of a
+// wave and keep their registers. The 128-thread columns (H = 1024) likewise: 1M x 1024 20.1 -> 19.4.
+constexpr int line_blocks(int T) { return T >= 512 || T < 64 ? 1 : 512 / T; }
+
 // ROE: measure the round-off |x - rint(x)| into roe[roeSlot]. The reference measures it on a
 // sample of iterations only, with a separate kernel build (kCarryFusedROE vs kCarryFused,
 // src/Gpu.cpp:592-596); the fused line pass without it runs about 0.8 us faster at 8M.
 // SPLIT (W = 2048 only): the first inverse and last forward radix-16 stages as INT8 tensor-core
 // GEMMs (owl_line_tc.cuh), the split-precision form of the line pass.
 template <int W, int R, int MODE, bool ROE = true, bool SPLIT = false>
-__global__ void __launch_bounds__(R * W / 16, (R * W / 16 == 256) ? 2 : 1)
+__global__ void __launch_bounds__(R * W / 16, line_blocks(R * W / 16))
     k_pass1(Args a, C* __restrict__ F, int32_t* __restrict__ words, int roeSlot, int flags, int tslot) {
   const uint32_t blk = blockIdx.x;
 #include "owl_pass1_body.inc"
@@ -259,7 +267,7 @@ template <int H, int R, int MODE, int VPT = 16, int MINB = 0>
 __global__ void __launch_bounds__(2 * H / VPT,
                                   MINB ? MINB
                                        : (((2 * H / VPT == 256) || (VPT == 8 && 2 * H / VPT == 512)) ? 2
-                                                                                                     : (H == 1280 ? 3 : 1)))
+                                                                                                     : (H == 1280 ? 3 : (2 * H / VPT == 128 ? 4 : 1))))
     k_pass2(Args a, C* __restrict__ F, const C* __restrict__ Fb, C* __restrict__ Fq, int tslot) {
   const uint32_t blk = blockIdx.x;
 #include "owl_pass2_body.inc"
