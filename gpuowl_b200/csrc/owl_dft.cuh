@@ -480,7 +480,9 @@ template <int N, int RL, int R1F = 0, int VPT = 16> struct Plan {
 // Read one by one where they are used, every one of these was an L2 round trip of its own per CTA, and
 // the two-level w_hN table two gathers of up to 32 wavefronts.
 struct LineTw {
-  static constexpr int M1 = 16, M2 = 20, RL = 24, LO = 27, HI = 43, HIB = 52, WT = 61, IWT = 62, LEN = 63;
+  static constexpr int M1 = 16, RL = 20, WT = 23, IWT = 24, LO = 25, HI = 41, HIB = 50, M2 = 59, LEN = 63;
+  // the entries that lines of w points use (up to 256 points: no HI, S = W/R1 <= 16 entries of LO)
+  static constexpr int used(int w) { return w <= 256 ? LO + (w == 256 ? 16 : 8) : (w <= 2048 ? M2 : LEN); }
 };
 
 // ---- The transform of two rows (lines or columns) whose middle exchanges stay inside a warp ----

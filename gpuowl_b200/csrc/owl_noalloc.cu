@@ -131,19 +131,15 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
   // the line groups' twist tables (line_tables; W here is below the width from which lanes pair)
   static_assert(kNoAllocMaxW < (uint32_t)owl::kPairMinW, "no-alloc widths");
   {
-    const uint32_t r1 = owl::plan_r1(W, 16 / kR), d1 = W / (r1 * owl::plan_m1(W, 16 / kR)),
-                   d2 = d1 / owl::plan_m2(W, 16 / kR), len = owl::LineTw::LEN;
+    const uint32_t r1 = owl::plan_r1(W, 16 / kR), d1 = W / (r1 * owl::plan_m1(W, 16 / kR)), len = owl::LineTw::LEN;
     for (uint32_t i = tid; i < H * len; i += nth) {
       const uint32_t x = i / (2 * len) * 2 + i % 2;
       const int e = (int)(i % (2 * len) / 2);
       const uint64_t m = e < owl::LineTw::M1 ? (e < (int)r1 ? (uint64_t)e * (W / r1) : 0u)
-                         : e < owl::LineTw::M2 ? (uint64_t)d1 << (e - owl::LineTw::M1)
-                         : e < owl::LineTw::RL ? (uint64_t)d2 << (e - owl::LineTw::M2)
-                         : e < owl::LineTw::LO ? (uint64_t)1 << (e - owl::LineTw::RL)
-                         : e < owl::LineTw::HI ? (uint64_t)(e - owl::LineTw::LO)
-                         : e < owl::LineTw::HIB ? (uint64_t)16 * (e - owl::LineTw::HI)
-                                                : a.hN + (uint64_t)16 * (e - owl::LineTw::HIB) - W;
-      if (e < owl::LineTw::WT) {
+                         : e < owl::LineTw::RL ? (uint64_t)d1 << (e - owl::LineTw::M1)
+                         : e < owl::LineTw::WT ? (uint64_t)1 << (e - owl::LineTw::RL)
+                         : e < owl::LineTw::HI ? (uint64_t)(e - owl::LineTw::LO) : 0;  // the rest is not used
+      if (e != owl::LineTw::WT && e != owl::LineTw::IWT) {
         const_cast<owl::C*>(a.twW)[twWn + i] = droot(a.hN, m * x);
       } else {
         const double X0 = (double)((step * (uint64_t)(2 * x)) % N) / N, X1 = (double)((step * (uint64_t)(2 * x + 1)) % N) / N;
