@@ -114,6 +114,15 @@ struct owl_plan {
     uint64_t lastUse;
   };
   std::vector<GraphEntry> graphs;
+  // the transforms of a product (up to its exit pass) as graphs, keyed by the two buffers and the timeout
+  struct MulGraph {
+    const int32_t* a;
+    const int32_t* b;
+    unsigned long long timeoutNs;
+    cudaGraphExec_t exec;  // null until the key is seen a second time
+    uint64_t lastUse;
+  };
+  std::vector<MulGraph> mulGraphs;
   uint64_t useClock = 0;
   // column variant (owl::COL_V16 / COL_V8 / COL_V16_OCC2) and the device copies of its stage
   // tables (COL_V16_OCC2 shares COL_V16's)
@@ -367,6 +376,10 @@ void pass1_out(owl_plan* p, int32_t* words, int flags, int fixedSlot = -1, int t
   ck(cudaGetLastError(), "fixup launch");
 }
 
+// Whether the line pass may be a programmatic dependent of the column pass (not of the split-precision
+// one: 8 us slower per iteration at 8M that way).
+bool pdl_line(const owl_plan* p) { return !(p->split & OWL_SPLIT_COLUMNS); }
+
 constexpr uint32_t kTsCap = 4096;  // launch-timestamp slots (profiled blocks of up to 2047 squarings)
 
 // Enqueues n squarings in -> out on the plan's stream: entry line pass, n x
@@ -385,9 +398,8 @@ void enqueue_square(owl_plan* p, int32_t* out, const int32_t* in, uint32_t n, ui
     ck(cudaMemsetAsync(p->args.tsStart, 0xff, cnt * sizeof(unsigned long long), p->stream), "memset ts");
     ck(cudaMemsetAsync(p->args.tsEnd, 0, cnt * sizeof(unsigned long long), p->stream), "memset ts");
   }
-  // the passes after the entry pass are programmatic dependents of the pass before them, except
-  // the line pass after the split-precision column pass (8 us slower per iteration at 8M that way)
-  const bool pdl = !(p->split & OWL_SPLIT_COLUMNS);
+  // the passes after the entry pass are programmatic dependents of the pass before them (pdl_line)
+  const bool pdl = pdl_line(p);
   pass1(p, owl::P1_IN, p->F1, const_cast<int32_t*>(in), 0, -1, ts());
   for (uint32_t k = 0; k < n; ++k) {
     pass2(p, owl::P2_SQUARE, p->F1, nullptr, nullptr, ts(), true);
@@ -522,6 +534,63 @@ void run_square(owl_plan* p, int32_t* out, const int32_t* in, uint32_t n, uint32
   auto& g = graph_for(p, out, in, n, flags, false);
   ck(cudaGraphLaunch(g.exec, p->stream), "cudaGraphLaunch");
   if (!(flags & OWL_SQ_NO_ROE)) { p->roePos = std::max(p->roePos, std::min(n, kRoeCap)); }
+}
+
+void drop_graphs(owl_plan* p) {
+  for (auto& g : p->graphs) { cudaGraphExecDestroy(g.exec); }
+  p->graphs.clear();
+  for (auto& g : p->mulGraphs) {
+    if (g.exec) { cudaGraphExecDestroy(g.exec); }
+  }
+  p->mulGraphs.clear();
+}
+
+// the transforms of io_a * in_b up to the spectrum of the product in F1
+void enqueue_mul(owl_plan* p, const int32_t* a, const int32_t* b) {
+  pass1(p, owl::P1_IN, p->F2, const_cast<int32_t*>(b), 0);
+  pass2(p, owl::P2_FWD, p->F2, nullptr, p->F2, -1, true);
+  pass1(p, owl::P1_IN, p->F1, const_cast<int32_t*>(a), 0, -1, -1, pdl_line(p));
+  pass2(p, owl::P2_MUL, p->F1, p->F2, nullptr, -1, true);
+}
+
+// enqueue_mul as one graph launch from the second call with the same buffers on: at 256K words a product
+// is bound by the host's six launches (21 us with several plans in turn)
+constexpr size_t kMulGraphMax = 4;
+void run_mul(owl_plan* p, const int32_t* a, const int32_t* b) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  ck(cudaStreamIsCapturing(p->stream, &cap), "cudaStreamIsCapturing");
+  if (cap != cudaStreamCaptureStatusNone) { return enqueue_mul(p, a, b); }
+  ++p->useClock;
+  auto it = std::find_if(p->mulGraphs.begin(), p->mulGraphs.end(), [&](const auto& g) {
+    return g.a == a && g.b == b && g.timeoutNs == p->args.timeoutNs;
+  });
+  if (it == p->mulGraphs.end()) {
+    if (p->mulGraphs.size() >= kMulGraphMax) {
+      auto lru = std::min_element(p->mulGraphs.begin(), p->mulGraphs.end(),
+                                  [](const auto& x, const auto& y) { return x.lastUse < y.lastUse; });
+      if (lru->exec) { cudaGraphExecDestroy(lru->exec); }
+      p->mulGraphs.erase(lru);
+    }
+    p->mulGraphs.push_back({a, b, p->args.timeoutNs, nullptr, p->useClock});
+    return enqueue_mul(p, a, b);
+  }
+  it->lastUse = p->useClock;
+  if (!it->exec) {
+    cudaGraph_t graph = nullptr;
+    ck(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
+    try {
+      enqueue_mul(p, a, b);
+    } catch (...) {
+      cudaStreamEndCapture(p->stream, &graph);
+      if (graph) { cudaGraphDestroy(graph); }
+      throw;
+    }
+    ck(cudaStreamEndCapture(p->stream, &graph), "cudaStreamEndCapture");
+    const cudaError_t e = cudaGraphInstantiate(&it->exec, graph, 0);
+    cudaGraphDestroy(graph);
+    ck(e, "cudaGraphInstantiate");
+  }
+  ck(cudaGraphLaunch(it->exec, p->stream), "cudaGraphLaunch");
 }
 
 void check_plan(const owl_plan* p) {
@@ -693,7 +762,7 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
 void plan_destroy(owl_plan* p) {
   DeviceGuard dg(p->device);
   if (p->stream) { cudaStreamSynchronize(p->stream); }
-  for (auto& g : p->graphs) { cudaGraphExecDestroy(g.exec); }
+  drop_graphs(p);
   for (int32_t* b : p->bufs) { cudaFree(b); }
   cudaFree(p->F1);
   cudaFree(p->F2);
@@ -880,8 +949,7 @@ int owl_plan_set_split(owl_plan* plan, int flags) {
     }
     DeviceGuard dg(plan->device);
     ck(cudaStreamSynchronize(plan->stream), "cudaStreamSynchronize");
-    for (auto& g : plan->graphs) { cudaGraphExecDestroy(g.exec); }
-    plan->graphs.clear();
+    drop_graphs(plan);
     plan->split = f;
   });
 }
@@ -895,8 +963,7 @@ int owl_plan_set_column_variant(owl_plan* plan, uint32_t variant) {
     }
     DeviceGuard dg(plan->device);
     ck(cudaStreamSynchronize(plan->stream), "cudaStreamSynchronize");
-    for (auto& g : plan->graphs) { cudaGraphExecDestroy(g.exec); }
-    plan->graphs.clear();
+    drop_graphs(plan);
     apply_col_variant(plan, cv);
   });
 }
@@ -1032,10 +1099,7 @@ int owl_modmul(owl_plan* plan, int32_t* io_a, const int32_t* in_b, int mul3) {
     check_buf(plan, io_a);
     check_buf(plan, in_b);
     DeviceGuard dg(plan->device);
-    pass1(plan, owl::P1_IN, plan->F2, const_cast<int32_t*>(in_b), 0);
-    pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2);
-    pass1(plan, owl::P1_IN, plan->F1, io_a, 0);
-    pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr);
+    run_mul(plan, io_a, in_b);
     pass1_out(plan, io_a, mul3 ? owl::FL_MUL3 : 0);
   });
 }
@@ -1053,25 +1117,27 @@ int owl_exp_mul(owl_plan* plan, int32_t* io_a, uint64_t h, const int32_t* in_b) 
       sync_and_check(plan);
       return;
     }
-    // left-to-right binary powering with the base's column spectrum kept in F2
+    // left-to-right binary powering with the base's column spectrum kept in F2; every pass waits for the
+    // one before it by itself (programmatic dependents)
+    const bool pdl = pdl_line(plan);
     pass1(plan, owl::P1_IN, plan->F2, io_a, 0);
-    pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2);
-    pass1(plan, owl::P1_IN, plan->F1, io_a, 0);
+    pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2, -1, true);
+    pass1(plan, owl::P1_IN, plan->F1, io_a, 0, -1, -1, pdl);
     int top = 63;
     while (!((h >> top) & 1)) { --top; }
     for (int b = top - 1; b >= 0; --b) {
-      pass2(plan, owl::P2_SQUARE, plan->F1, nullptr, nullptr);
-      pass1(plan, owl::P1_FUSED, plan->F1, nullptr, 0);
+      pass2(plan, owl::P2_SQUARE, plan->F1, nullptr, nullptr, -1, true);
+      pass1(plan, owl::P1_FUSED, plan->F1, nullptr, 0, -1, -1, pdl);
       if ((h >> b) & 1) {
-        pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr);
-        pass1(plan, owl::P1_FUSED, plan->F1, nullptr, 0);
+        pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr, -1, true);
+        pass1(plan, owl::P1_FUSED, plan->F1, nullptr, 0, -1, -1, pdl);
       }
     }
     // times B
-    pass1(plan, owl::P1_IN, plan->F2, const_cast<int32_t*>(in_b), 0);
-    pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2);
-    pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr);
-    pass1_out(plan, io_a, 0);
+    pass1(plan, owl::P1_IN, plan->F2, const_cast<int32_t*>(in_b), 0, -1, -1, true);
+    pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2, -1, true);
+    pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr, -1, true);
+    pass1_out(plan, io_a, 0, -1, -1, pdl);
     sync_and_check(plan);
   });
 }
