@@ -33,9 +33,6 @@ __device__ __forceinline__ uint32_t ld_acquire(const uint32_t* p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release(uint32_t* p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 // a carry word, read and written by single threads of different CTAs without further ordering: each
 // word carries its own validity (its tag), so no fence or flag orders it against other data
 __device__ __forceinline__ long long ld_relaxed(const long long* p) {
