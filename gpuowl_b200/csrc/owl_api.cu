@@ -610,11 +610,14 @@ void sync_and_check(owl_plan* p) {
   uint32_t err = 0;
   ck(cudaMemcpy(&err, &p->args.ctl->error, sizeof(err), cudaMemcpyDeviceToHost), "read error word");
   if (err) {
-    // reset the carry-chain state so that the plan stays usable
+    // reset the carry-chain state so that the plan stays usable: on the plan's own stream (non-blocking, so
+    // the default stream orders nothing before its launches), the tag of the ticket counter and the carry
+    // words together, before anything of the plan runs again
     uint32_t G = p->H / kR;
-    ck(cudaMemset(p->args.ctl, 0, sizeof(owl::Ctl)), "reset ctl");
-    ck(cudaMemset(p->args.flags, 0, G * sizeof(uint32_t)), "reset flags");
-    ck(cudaMemset(p->args.shuttle, 0, (size_t)G * p->W * sizeof(long long)), "reset carry words");
+    ck(cudaMemsetAsync(p->args.ctl, 0, sizeof(owl::Ctl), p->stream), "reset ctl");
+    ck(cudaMemsetAsync(p->args.flags, 0, G * sizeof(uint32_t), p->stream), "reset flags");
+    ck(cudaMemsetAsync(p->args.shuttle, 0, (size_t)G * p->W * sizeof(long long), p->stream), "reset carry words");
+    ck(cudaStreamSynchronize(p->stream), "cudaStreamSynchronize");
     fail(OWL_ERR_TIMEOUT, "device-side carry wait timed out");
   }
 }
@@ -712,7 +715,8 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
     p->tcB = reinterpret_cast<const unsigned char*>(dbase + put(tcB.data(), tcB.size()));
   }
   if (!tc1B.empty()) { p->args.tc1B = reinterpret_cast<const unsigned char*>(dbase + put(tc1B.data(), tc1B.size())); }
-  ck(cudaMemcpy(p->tableMem, host.data(), bytes, cudaMemcpyHostToDevice), "upload tables");
+  // on the plan's own stream (see sync_and_check)
+  ck(cudaMemcpyAsync(p->tableMem, host.data(), bytes, cudaMemcpyHostToDevice, p->stream), "upload tables");
 
   // FFT work buffers
   ck(cudaMalloc(&p->F1, (size_t)p->hN * sizeof(C)), "cudaMalloc(F1)");
@@ -726,7 +730,8 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
                   2 * owl::kPendingCap * sizeof(long long) + 2 * kTsCap * sizeof(unsigned long long) +
                   kRoeCap * sizeof(float) + 64 * sizeof(int32_t) + sizeof(unsigned long long) + sizeof(int);
   ck(cudaMalloc(&p->scratch, sbytes), "cudaMalloc(scratch)");
-  ck(cudaMemset(p->scratch, 0, sbytes), "memset(scratch)");
+  ck(cudaMemsetAsync(p->scratch, 0, sbytes, p->stream), "memset(scratch)");
+  ck(cudaStreamSynchronize(p->stream), "cudaStreamSynchronize");
   char* cur = static_cast<char*>(p->scratch);
   p->args.shuttle = carve<long long>(cur, (size_t)G * W);
   p->args.flags = carve<uint32_t>(cur, G);

@@ -1,0 +1,64 @@
+"""What the host code enqueues, on a recording stand-in for the CUDA runtime (tests/fake_cuda): streams,
+order, launch attributes and graphs of the API's calls, without a GPU."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "gpuowl_b200", "csrc")
+FAKE = os.path.join(ROOT, "tests", "fake_cuda")
+NVCC = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+
+
+@pytest.fixture(scope="module")
+def host_log(tmp_path_factory):
+    if not os.path.exists(NVCC):
+        pytest.skip("no nvcc")
+    d = tmp_path_factory.mktemp("host_log")
+    src = d / "csrc"
+    shutil.copytree(CSRC, src)
+    for body in ("owl_pass1_body.inc", "owl_pass2_body.inc"):  # the kernels do not run: 20 s instead of minutes
+        (src / body).write_text("")
+    exe = str(d / "host_log")
+    subprocess.run([NVCC, "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-w", "-cudart", "none",
+                    "--expt-relaxed-constexpr", "-I", str(src), "-I", os.path.join(ROOT, "include"), "-o", exe,
+                    os.path.join(FAKE, "host_log.cu"), os.path.join(FAKE, "fake_cuda.cpp")],
+                   check=True, capture_output=True)
+
+    def run(*args):
+        r = subprocess.run([exe] + [str(a) for a in args], capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, (r.stdout[-2000:], r.stderr[-2000:])
+        sections, name = {}, ""
+        for line in r.stdout.splitlines():
+            if line.startswith("== "):
+                name = line[3:]
+                while name in sections:
+                    name += "'"
+                sections[name] = []
+            else:
+                sections.setdefault(name, []).append(line)
+        return sections
+    return run
+
+
+def test_a_new_plan_is_ready(host_log):
+    """Tables and cleared scratch are there when the call returns: the plan's stream does not wait for the
+    default stream, on which an upload or a memset may still be under way."""
+    ops = host_log("create")["create"]
+    assert [x for x in ops if x.startswith("stream ")] == ["stream 1 non-blocking"]
+    moves = [i for i, x in enumerate(ops) if x.startswith(("memset", "copy"))]
+    assert len(moves) >= 2 and all(ops[i] in ("memset stream=1", "copy stream=1") for i in moves), ops
+    assert "wait stream=1" in ops[moves[-1]:], ops
+
+
+def test_reset_after_a_timeout_is_ordered(host_log):
+    """The control word and the carry words of a plan whose wait ran out are cleared on its own stream, and
+    the call returns once they are (a launch between the two would take old carry words for new ones)."""
+    ops = host_log("reset")["sync"]
+    assert ops[-1] == "status -4"
+    sets = [i for i, x in enumerate(ops) if x.startswith("memset")]
+    assert len(sets) >= 2 and all(ops[i] == "memset stream=1" for i in sets), ops
+    assert "wait stream=1" in ops[sets[-1]:], ops
