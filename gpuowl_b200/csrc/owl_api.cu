@@ -1123,7 +1123,7 @@ int owl_exp_mul(owl_plan* plan, int32_t* io_a, uint64_t h, const int32_t* in_b) 
       return;
     }
     // left-to-right binary powering with the base's column spectrum kept in F2; every pass waits for the
-    // one before it by itself (programmatic dependents)
+    // one before it by itself (programmatic dependents), but for the last product
     const bool pdl = pdl_line(plan);
     pass1(plan, owl::P1_IN, plan->F2, io_a, 0);
     pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2, -1, true);
@@ -1141,7 +1141,9 @@ int owl_exp_mul(owl_plan* plan, int32_t* io_a, uint64_t h, const int32_t* in_b) 
     // times B
     pass1(plan, owl::P1_IN, plan->F2, const_cast<int32_t*>(in_b), 0, -1, -1, true);
     pass2(plan, owl::P2_FWD, plan->F2, nullptr, plan->F2, -1, true);
-    pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr, -1, true);
+    // a plain launch: the product pass takes F2 as read-only for as long as it runs, and the pass before
+    // it writes F2 (elsewhere another pass lies between the two)
+    pass2(plan, owl::P2_MUL, plan->F1, plan->F2, nullptr, -1, false);
     pass1_out(plan, io_a, 0, -1, -1, pdl);
     sync_and_check(plan);
   });

@@ -62,3 +62,18 @@ def test_reset_after_a_timeout_is_ordered(host_log):
     sets = [i for i, x in enumerate(ops) if x.startswith("memset")]
     assert len(sets) >= 2 and all(ops[i] == "memset stream=1" for i in sets), ops
     assert "wait stream=1" in ops[sets[-1]:], ops
+
+
+@pytest.mark.parametrize("W,H,split", [(64, 64, 0), (2048, 64, 0), (64, 2560, 0), (64, 2048, 1), (64, 2560, 1)])
+def test_a_kept_spectrum_is_complete_before_the_pass_that_reads_it_starts(host_log, W, H, split):
+    """The product pass declares the kept spectrum read-only while it runs, so it must not be a programmatic
+    dependent of the pass that writes it."""
+    log = host_log("power", W, H, split)
+    for name, muls in (("power", 5), ("product", 1), ("product'", 1)):  # 0xb5 has four bits below its top
+        k = [x for x in log[name] if x.startswith("launch k_pass")]
+        mode = [int(x.split("<")[1].split(">")[0].split(",")[2]) for x in k]
+        at = [i for i, x in enumerate(k) if x.startswith("launch k_pass2") and mode[i] == 2]
+        assert len(at) == muls, k
+        for i in at:
+            after_writer = k[i - 1].startswith("launch k_pass2") and mode[i - 1] == 1
+            assert not (after_writer and "pdl=1" in k[i]), k[i - 1:i + 1]
