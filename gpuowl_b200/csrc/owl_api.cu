@@ -104,12 +104,14 @@ struct owl_plan {
   int* eq = nullptr;
   uint32_t roePos = 0;
   std::vector<int32_t*> bufs;
-  // squaring blocks captured as CUDA graphs, keyed by (in, out, n, flags, with events)
+  // squaring blocks captured as CUDA graphs, keyed by (in, out, n, flags, with events, timeout): a captured
+  // launch keeps the arguments it was captured with
   struct GraphEntry {
     const int32_t* in;
     int32_t* out;
     uint32_t n, flags;
     bool profiled;
+    unsigned long long timeoutNs;
     cudaGraphExec_t exec;
     uint64_t lastUse;
   };
@@ -497,7 +499,8 @@ owl_plan::GraphEntry& graph_for(owl_plan* p, int32_t* out, const int32_t* in, ui
                                 bool profiled) {
   ++p->useClock;
   for (auto& g : p->graphs) {
-    if (g.in == in && g.out == out && g.n == n && g.flags == flags && g.profiled == profiled) {
+    if (g.in == in && g.out == out && g.n == n && g.flags == flags && g.profiled == profiled &&
+        g.timeoutNs == p->args.timeoutNs) {
       g.lastUse = p->useClock;
       return g;
     }
@@ -508,7 +511,7 @@ owl_plan::GraphEntry& graph_for(owl_plan* p, int32_t* out, const int32_t* in, ui
     cudaGraphExecDestroy(lru->exec);
     p->graphs.erase(lru);
   }
-  owl_plan::GraphEntry g{in, out, n, flags, profiled, nullptr, p->useClock};
+  owl_plan::GraphEntry g{in, out, n, flags, profiled, p->args.timeoutNs, nullptr, p->useClock};
   cudaGraph_t graph = nullptr;
   ck(cudaStreamBeginCapture(p->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   try {
@@ -1281,8 +1284,17 @@ struct owl_batch {
   std::vector<owl_plan*> plans;
   cudaEvent_t fork = nullptr, done = nullptr;
   std::vector<cudaEvent_t> joins;
+  struct Settings {  // of a plan, as captured
+    unsigned long long timeoutNs;
+    uint32_t split;
+    int colVariant;
+    bool operator==(const Settings& o) const {
+      return timeoutNs == o.timeoutNs && split == o.split && colVariant == o.colVariant;
+    }
+  };
   struct Entry {
     std::vector<int32_t*> bufs;
+    std::vector<Settings> settings;
     uint32_t n, flags;
     cudaGraphExec_t exec;
   };
@@ -1304,8 +1316,10 @@ void batch_destroy(owl_batch* b) {
 
 cudaGraphExec_t batch_graph(owl_batch* b, int32_t* const* bufs, uint32_t n, uint32_t flags) {
   std::vector<int32_t*> key(bufs, bufs + b->plans.size());
+  std::vector<owl_batch::Settings> settings;
+  for (const owl_plan* p : b->plans) { settings.push_back({p->args.timeoutNs, p->split, p->colVariant}); }
   for (auto& g : b->graphs) {
-    if (g.n == n && g.flags == flags && g.bufs == key) { return g.exec; }
+    if (g.n == n && g.flags == flags && g.bufs == key && g.settings == settings) { return g.exec; }
   }
   if (b->graphs.size() >= 4) {
     cudaGraphExecDestroy(b->graphs.front().exec);
@@ -1366,7 +1380,7 @@ cudaGraphExec_t batch_graph(owl_batch* b, int32_t* const* bufs, uint32_t n, uint
   cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
   ck(e, "cudaGraphInstantiate");
-  b->graphs.push_back({key, n, flags, exec});
+  b->graphs.push_back({key, settings, n, flags, exec});
   return exec;
 }
 

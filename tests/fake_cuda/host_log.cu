@@ -1,7 +1,7 @@
 // host_log.cu -- runs calls of the library's C ABI on the recording runtime (fake_cuda.cpp) and prints what
 // they enqueue, for tests/test_host_launches.py. Compiled with the pass bodies left empty.
 //
-// TEST INFRASTRUCTURE ONLY. Usage: host_log create | reset | timeouts | power W H split
+// TEST INFRASTRUCTURE ONLY. Usage: host_log create | reset | timeouts | settings | power W H split
 #include "owl_api.cu"
 
 #include <cstdlib>
@@ -75,6 +75,21 @@ int main(int argc, char** argv) {
       mark("batch");
       must(owl_batch_square(batch, bufs, 3, 0));
     }
+    mark("end");
+  } else if (what == "settings") {
+    owl_plan* p = plan(64, 2048);
+    int32_t* a = buf(p);
+    owl_batch* batch = nullptr;
+    must(owl_batch_create(0, 1, &p, &batch));
+    mark("plain");
+    must(owl_batch_square(batch, &a, 3, 0));
+    must(owl_plan_set_split(p, OWL_SPLIT_COLUMNS));
+    mark("split");
+    must(owl_batch_square(batch, &a, 3, 0));
+    must(owl_plan_set_split(p, 0));
+    must(owl_plan_set_column_variant(p, OWL_COL_V8));
+    mark("variant");
+    must(owl_batch_square(batch, &a, 3, 0));
     mark("end");
   } else if (what == "power" && argc == 5) {
     owl_plan* p = plan((uint32_t)std::atoi(argv[2]), (uint32_t)std::atoi(argv[3]), (uint32_t)std::atoi(argv[4]));

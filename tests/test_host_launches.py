@@ -77,3 +77,28 @@ def test_a_kept_spectrum_is_complete_before_the_pass_that_reads_it_starts(host_l
         for i in at:
             after_writer = k[i - 1].startswith("launch k_pass2") and mode[i - 1] == 1
             assert not (after_writer and "pdl=1" in k[i]), k[i - 1:i + 1]
+
+
+def test_cached_graphs_follow_the_wait_limit(host_log):
+    """A block, a profiled block, a product and a batch that run as cached graphs wait as long as the last
+    set limit says, and a limit that comes back finds its graphs again."""
+    log = host_log("timeouts")
+    graphs = []
+    for name, batch, limit in (("limit 7", "batch", 7), ("limit 9", "batch'", 9), ("limit 7'", "batch''", 7)):
+        k = [x for x in log[name] if x.startswith("launch k_pass")]
+        assert len(k) > 70 and all(" timeout=%d " % limit in x + " " for x in k), (name, k[:2])
+        kb = [x for x in log[batch] if x.startswith("launch k_pass")]
+        assert {x.split("timeout=")[1].split()[0] for x in kb} == {"%d,2000000000" % limit, str(limit + 1)}, kb[:2]
+        graphs.append([x for x in log[name] + log[batch] if x.startswith("graph ")])
+    assert graphs[0] != graphs[1]
+    # a product becomes a graph on the second call with its buffers, so limit 7 ran one on its first call here
+    assert set(graphs[0]) <= set(graphs[2])
+
+
+def test_batch_graph_follows_the_plans_settings(host_log):
+    """A batch that was captured before a plan's split form or column variant changed is captured again."""
+    log = host_log("settings")
+    runs = [[x.split()[1] for x in log[s] if x.startswith("launch k_pass2")] for s in ("plain", "split", "variant")]
+    assert not any("k_pass2_tc" in x for x in runs[0])
+    assert any("k_pass2_tc" in x for x in runs[1])
+    assert any(x.startswith("k_pass2") and ",8," in x for x in runs[2])
