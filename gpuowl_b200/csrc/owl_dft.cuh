@@ -480,9 +480,11 @@ template <int N, int RL, int R1F = 0, int VPT = 16> struct Plan {
 // Read one by one where they are used, every one of these was an L2 round trip of its own per CTA, and
 // the two-level w_hN table two gathers of up to 32 wavefronts.
 struct LineTw {
-  static constexpr int M1 = 16, RL = 20, WT = 23, IWT = 24, LO = 25, HI = 41, HIB = 50, M2 = 59, LEN = 63;
-  // the entries that lines of w points use (up to 256 points: no HI, S = W/R1 <= 16 entries of LO)
-  static constexpr int used(int w) { return w <= 256 ? LO + (w == 256 ? 16 : 8) : (w <= 2048 ? M2 : LEN); }
+  static constexpr int M1 = 16, RL = 20, WT = 23, IWT = 24, LO = 25, HI = 41, HIB = 50, M2 = 59;
+  // length of the record of lines of w points (up to 256 points: no HI, S = W/R1 <= 16 entries of LO)
+  __host__ __device__ static constexpr int len(int w) {
+    return w <= 256 ? LO + (w == 256 ? 16 : 8) : (w <= 2048 ? M2 : M2 + 4);
+  }
 };
 
 // ---- The transform of two rows (lines or columns) whose middle exchanges stay inside a warp ----

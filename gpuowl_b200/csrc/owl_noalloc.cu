@@ -70,7 +70,7 @@ struct Layout {
 Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   const uint32_t hN = W * H, G = H / kR;
   const int vH = owl::col_vpt(owl::COL_V16);  // the default column variant's kernels
-  const int twWn = owl::tw_offsets((int)W, 16 / kR).total + (int)H * owl::LineTw::LEN;
+  const int twWn = owl::tw_offsets((int)W, 16 / kR).total + (int)H * owl::LineTw::len((int)W);
   const int twHn = owl::tw_offsets((int)H, vH / 2, 0, vH).total + (int)H / (vH / 2);
   Layout L{};
   size_t o = 0;
@@ -131,7 +131,7 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
   // the line groups' twist tables (line_tables; W here is below the width from which lanes pair)
   static_assert(kNoAllocMaxW < (uint32_t)owl::kPairMinW, "no-alloc widths");
   {
-    const uint32_t r1 = owl::plan_r1(W, 16 / kR), d1 = W / (r1 * owl::plan_m1(W, 16 / kR)), len = owl::LineTw::LEN;
+    const uint32_t r1 = owl::plan_r1(W, 16 / kR), d1 = W / (r1 * owl::plan_m1(W, 16 / kR)), len = (uint32_t)owl::LineTw::len((int)W);
     for (uint32_t i = tid; i < H * len; i += nth) {
       const uint32_t x = i / (2 * len) * 2 + i % 2;
       const int e = (int)(i % (2 * len) / 2);

@@ -54,29 +54,41 @@ inline HostC root(uint64_t n, uint64_t k) {
   return HostC{(double)c, (double)-s};
 }
 
-// Many roots of one order: w_n^k as a product of two tabulated factors, taken in long double and rounded
-// once (sine and cosine of every entry would make the line groups' records the longest part of making
-// a plan: 105K roots at 8M words).
+// Many roots of one order n (a multiple of 8): w_n^k as a product of two tabulated factors, taken in long
+// double and rounded once (sine and cosine of every entry would make the line groups' records the longest
+// part of making a plan: 100K roots at 8M words). The factors, rounded, are the kernels' two-level table.
 class Roots {
  public:
-  explicit Roots(uint64_t n) : n_(n) {
+  explicit Roots(uint32_t n) : n8_(n / 8) {
     while ((1ull << (2 * sh_)) < n) { ++sh_; }
-    lo_.resize(1ull << sh_);
-    hi_.resize((n >> sh_) + 1);
-    for (uint64_t i = 0; i < lo_.size(); ++i) { root_ld(n, i, &lo_[i].first, &lo_[i].second); }
-    for (uint64_t i = 0; i < hi_.size(); ++i) { root_ld(n, i << sh_, &hi_[i].first, &hi_[i].second); }
+    lo_.resize(1u << sh_);
+    hi_.resize((n - 1) / (1u << sh_) + 1);
+    for (uint32_t i = 0; i < lo_.size(); ++i) { root_ld(n, i, &lo_[i].first, &lo_[i].second); }
+    for (uint32_t i = 0; i < hi_.size(); ++i) { root_ld(n, (uint64_t)i << sh_, &hi_[i].first, &hi_[i].second); }
+    for (uint32_t i = 0; i < 8; ++i) { eighth_[i] = root(8, i); }
   }
-  HostC at(uint64_t k) const {
-    k %= n_;
-    if (8 * k % n_ == 0) { return root(n_, k); }  // zeros and equal parts exactly
-    const auto &a = lo_[k & ((1ull << sh_) - 1)], &b = hi_[k >> sh_];
+  // k < n
+  HostC at(uint32_t k) const {
+    if (k % n8_ == 0) { return eighth_[k / n8_]; }  // zeros and equal parts exactly
+    const auto &a = lo_[k & ((1u << sh_) - 1)], &b = hi_[k >> sh_];
     return HostC{(double)(a.first * b.first - a.second * b.second), -(double)(a.first * b.second + a.second * b.first)};
   }
+  uint32_t lo_shift() const { return (uint32_t)sh_; }
+  std::vector<HostC> lo() const { return rounded(lo_); }  // w_n^i
+  std::vector<HostC> hi() const { return rounded(hi_); }  // w_n^(i << lo_shift())
 
  private:
-  uint64_t n_;
+  using Table = std::vector<std::pair<long double, long double>>;  // cos, sin
+  static std::vector<HostC> rounded(const Table& t) {
+    std::vector<HostC> r;
+    r.reserve(t.size());
+    for (const auto& x : t) { r.push_back({(double)x.first, (double)-x.second}); }
+    return r;
+  }
+  uint32_t n8_;
   int sh_ = 0;
-  std::vector<std::pair<long double, long double>> lo_, hi_;  // cos, sin
+  Table lo_, hi_;
+  HostC eighth_[8];
 };
 
 inline bool is_pow2(uint32_t x) { return x && !(x & (x - 1)); }
@@ -137,39 +149,55 @@ inline int default_col_variant(uint32_t W, uint32_t H) {
 // upper half of their sub-transform, conj(w_2R1^k) for w_2R1^k (and the twist's entry for the same row).
 inline bool line_pairs(uint32_t W) { return W >= 512; }
 
-// the line pass's tables: the stage tables of W points, then the record of every line group (LineTw);
-// wt2 and iwt2: the weights of the words of every line
-inline std::vector<HostC> line_tables(uint32_t W, uint32_t H, const double* wt2, const double* iwt2) {
-  const uint32_t rl = 8;
-  const uint64_t hN = (uint64_t)W * H;
-  const Roots roots(hN);
+// the entries of a line group's record (LineTw) that lines of W points read, and their exponents: entry
+// `at` of line x is w_hN^(m x)
+struct LineEntry {
+  int at;
+  uint32_t m;
+};
+inline std::vector<LineEntry> line_entries(uint32_t W, uint32_t H) {
+  const uint32_t hN = W * H, rl = 8, r1 = plan_r1(W, rl), m1 = plan_m1(W, rl), m2 = plan_m2(W, rl);
+  const uint32_t S = W / r1, d1 = S / m1, d2 = d1 / m2;
+  const bool pairs = line_pairs(W);
+  std::vector<LineEntry> v;
+  auto put = [&](int at, uint32_t m) { v.push_back({at, m % hN}); };
+  for (uint32_t r = 0; r < r1; ++r) { put((int)r, r * S); }
+  // d^(2^i) for the table rows 2^i < R that a stage of radix R reads
+  for (int i = 0; (2u << i) <= m1; ++i) { put(LineTw::M1 + i, pairs && (2u << i) == m1 ? W / 32 * 31 : d1 << i); }
+  for (int i = 0; (2u << i) <= m2; ++i) { put(LineTw::M2 + i, d2 << i); }
+  for (int i = 0; (2u << i) <= rl; ++i) { put(LineTw::RL + i, 1u << i); }
+  for (uint32_t j = 0; j < std::min(S, 16u); ++j) { put(LineTw::LO + (int)j, j); }
+  for (uint32_t j = 0; pairs && j <= S / 32; ++j) {
+    put(LineTw::HI + (int)j, 16 * j);
+    put(LineTw::HIB + (int)j, hN + 16 * j - W);
+  }
+  return v;
+}
+
+// the line pass's tables: the stage tables of W points, then the record of every line group (LineTw; entries
+// that lines of this width do not read are 0); wt2 and iwt2: the weights of the words of every line
+inline std::vector<HostC> line_tables(uint32_t W, uint32_t H, const Roots& roots, const double* wt2,
+                                      const double* iwt2) {
+  const uint32_t rl = 8, hN = W * H, len = (uint32_t)LineTw::len((int)W);
   std::vector<HostC> t = stage_tables(W, rl, 0, 16, true);
   const TwOffsets o = tw_offsets((int)W, (int)rl);
-  const uint32_t r1 = plan_r1(W, rl), m1 = plan_m1(W, rl), m2 = plan_m2(W, rl);
-  const bool pairs = line_pairs(W);
-  if (pairs) {
+  const uint32_t r1 = plan_r1(W, rl), m1 = plan_m1(W, rl);
+  if (line_pairs(W)) {
     for (uint32_t k = 0; k < r1; ++k) {
       HostC& w = t[o.aM1 + m1 / 2 * r1 + k];
       w.y = -w.y;
     }
   }
   const size_t at = t.size();
-  t.resize(at + (size_t)H * LineTw::LEN);
+  t.resize(at + (size_t)H * len);
+  const std::vector<LineEntry> entries = line_entries(W, H);
+  std::vector<uint32_t> k(entries.size(), 0);  // m x mod hN
   for (uint32_t x = 0; x < H; ++x) {
-    HostC* e = t.data() + at + (size_t)(x / 2) * (2 * LineTw::LEN) + x % 2;
-    auto put = [&](int i, uint64_t m) { e[2 * i] = roots.at(m * x); };
-    for (uint32_t r = 0; r < 16; ++r) { put((int)r, r < r1 ? r * (W / r1) : 0); }
-    const uint32_t d1 = W / (r1 * m1), d2 = d1 / m2;
-    for (int i = 0; i < 4; ++i) {
-      put(LineTw::M1 + i, (uint64_t)d1 << i);
-      put(LineTw::M2 + i, (uint64_t)d2 << i);
-      if (i < 3) { put(LineTw::RL + i, 1u << i); }
-      if (pairs && (2u << i) == m1) { put(LineTw::M1 + i, W / 32 * 31); }
-    }
-    for (uint32_t j = 0; j < 16; ++j) { put(LineTw::LO + (int)j, j); }
-    for (uint32_t j = 0; j < (pairs ? 9u : 1u); ++j) {
-      put(LineTw::HI + (int)j, 16 * j);
-      put(LineTw::HIB + (int)j, hN + 16 * j - W);  // mod hN
+    HostC* e = t.data() + at + (size_t)(x / 2) * (2 * len) + x % 2;
+    for (size_t i = 0; i < entries.size(); ++i) {
+      e[2 * entries[i].at] = roots.at(k[i]);
+      k[i] += entries[i].m;
+      if (k[i] >= hN) { k[i] -= hN; }
     }
     e[2 * LineTw::WT] = HostC{wt2[2 * x], wt2[2 * x + 1]};
     e[2 * LineTw::IWT] = HostC{iwt2[2 * x], iwt2[2 * x + 1]};
@@ -237,15 +265,15 @@ inline std::vector<uint32_t> word_masks(uint32_t E, uint32_t W, uint32_t H, cons
   }
   auto groups = [&](uint32_t g0, uint32_t g1) {
     for (uint32_t g = g0; g < g1; ++g) {
-      uint32_t xl[2 * R];
-      for (uint32_t i = 0; i < 2 * R; ++i) { xl[i] = x2[2 * R * g + i]; }
+      const uint32_t* xl = x2 + 2 * R * g;  // i = 2 ll + e
       for (uint32_t th = 0; th < T; ++th) {
         uint32_t big = 0, wrap = 0;
-        for (uint32_t r = 0; r < RL; ++r) {
-          for (uint32_t i = 0; i < 2 * R; ++i) {  // i = 2 ll + e
-            const uint32_t X = xt[th * RL + r] + xl[i], w = X >= N;
-            wrap |= w << (r * 2 * R + i);
-            big |= (uint32_t)(X - (N & (0u - w)) < em) << (r * 2 * R + i);
+        for (uint32_t r = RL; r-- > 0;) {  // from the top bit down
+          const uint32_t x = xt[th * RL + r];
+          for (uint32_t i = 2 * R; i-- > 0;) {
+            const uint32_t X = x + xl[i];
+            wrap = 2 * wrap + (X >= N);
+            big = 2 * big + (X < em) + (X - N < em);  // unsigned: at most one of the two
           }
         }
         m[2 * ((size_t)g * T + th)] = big;
@@ -253,7 +281,7 @@ inline std::vector<uint32_t> word_masks(uint32_t E, uint32_t W, uint32_t H, cons
       }
     }
   };
-  // 2 ns a word: 40 ms at 20M words on one thread
+  // 1.3 ns a word: 27 ms at 20M words on one thread
   const unsigned nt = N < (1u << 20) ? 1u : std::max(1u, std::min(std::thread::hardware_concurrency(), 8u));
   std::vector<std::thread> pool;
   pool.reserve(nt);
@@ -279,16 +307,13 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
   t.hN = W * H;
   t.N = 2 * W * H;
   const uint32_t N = t.N;
-  t.loShift = (log2u(t.hN) + 1) / 2;
+  const Roots roots(t.hN);
+  t.loShift = roots.lo_shift();
   t.twH = col_stage_tables(H, COL_V16);
   t.rootH.resize(H);
   for (uint32_t i = 0; i < H; ++i) { t.rootH[i] = root(H, i); }
-  uint32_t S = 1u << t.loShift;
-  t.twLo.resize(S);
-  for (uint32_t i = 0; i < S; ++i) { t.twLo[i] = root(t.hN, i); }
-  uint32_t nHi = (t.hN + S - 1) / S;
-  t.twHi.resize(nHi);
-  for (uint32_t i = 0; i < nHi; ++i) { t.twHi[i] = root(t.hN, (uint64_t)i * S); }
+  t.twLo = roots.lo();
+  t.twHi = roots.hi();
 
   const uint64_t step = N - (E % N);
   t.x1.resize(W);
@@ -314,7 +339,7 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
     t.wt2[i] = (double)exp2l((long double)X / N);
     t.iwt2[i] = (double)(exp2l(-(long double)X / N) * norm);
   }
-  t.twW = line_tables(W, H, t.wt2.data(), t.iwt2.data());
+  t.twW = line_tables(W, H, roots, t.wt2.data(), t.iwt2.data());
   t.p1masks = word_masks(E, W, H, t.x1.data(), t.x2.data());
   return t;
 }

@@ -12,7 +12,8 @@
 // tensor cores. With OWL_EMU_NO_ROE=1 the fused line passes run the build without the round-off
 // measurement. OWL_EMU_COL=<v> runs the
 // column pass's variant v (owl::COL_V16 / COL_V8 / COL_V16_OCC2) with its stage tables. With
-// OWL_EMU_GROUP=1 the line passes run the grouped kernel of a batch (one plan as the group).
+// OWL_EMU_GROUP=1 the line passes run the grouped kernel of a batch (one plan as the group). With
+// OWL_EMU_POISON=1 the entries of the line groups' records that no lines of this width should read are NaN.
 // Output: one line "roe <max>" then one line of nWords hex u32 (little-endian order).
 #define OWL_EMU 1
 #include <algorithm>
@@ -59,6 +60,15 @@ std::vector<C> toC(const std::vector<HostC>& v) {
 void init(EmuPlan& p, uint32_t E, uint32_t W, uint32_t H) {
   p.t = make_tables(E, W, H);
   p.twW = toC(p.t.twW);
+  if (std::getenv("OWL_EMU_POISON")) {
+    const size_t len = LineTw::len((int)W), base = p.twW.size() - H * len;
+    std::vector<char> read(len, 0);
+    read[LineTw::WT] = read[LineTw::IWT] = 1;
+    for (const LineEntry& e : line_entries(W, H)) { read.at(e.at) = 1; }
+    for (size_t i = 0; i < H * len; ++i) {
+      if (!read[i % (2 * len) / 2]) { p.twW[base + i] = make_double2(std::nan(""), std::nan("")); }
+    }
+  }
   p.twH = toC(p.t.twH);
   p.rootH = toC(p.t.rootH);
   p.twLo = toC(p.t.twLo);
@@ -205,6 +215,7 @@ void pass1(EmuPlan& p, int mode, C* F, int32_t* words, int flags) {
     case 512: p1w<512>(p, mode, F, words, flags); break;
     case 1024: p1w<1024>(p, mode, F, words, flags); break;
     case 2048: p1w<2048>(p, mode, F, words, flags); break;
+    case 4096: p1w<4096>(p, mode, F, words, flags); break;
     default: throw std::runtime_error("emu W");
   }
   if (mode == P1_OUT) {
@@ -226,6 +237,8 @@ void pass2(EmuPlan& p, int mode, C* F, const C* Fb, C* Fq) {
     case 128: p2h<128>(p, mode, F, Fb, Fq); break;
     case 256: p2h<256>(p, mode, F, Fb, Fq); break;
     case 512: p2h<512>(p, mode, F, Fb, Fq); break;
+    case 1024: p2h<1024>(p, mode, F, Fb, Fq); break;
+    case 4096: p2h<4096>(p, mode, F, Fb, Fq); break;
     case 640: p2h<640>(p, mode, F, Fb, Fq); break;
     case 1280: p2h<1280>(p, mode, F, Fb, Fq); break;
     case 2560: p2h<2560>(p, mode, F, Fb, Fq); break;

@@ -22,6 +22,15 @@ def test_emulated_edges(emu, oracle, W, H, n, flags):  # noqa: F811
     assert np.array_equal(got, oracle.gmp_square(E, random_words(E, 9), n, ll=bool(flags & 2)))
 
 
+@pytest.mark.parametrize("W", [64, 128, 256, 512, 1024, 2048, 4096])
+def test_emulated_records_hold_what_lines_read(emu, oracle, W):  # noqa: F811
+    """Making a plan computes only the entries of a line group's record that lines of its width read: with
+    every other entry NaN the words are still GMP's."""
+    E = exponent(W, 64)
+    _, got = run(emu, "square", E, W, 64, 2, 0, 9, OWL_EMU_POISON="1")
+    assert np.array_equal(got, oracle.gmp_square(E, random_words(E, 9), 2))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("W,H", EDGES)
 def test_edges_vs_gmp(oracle, W, H):
