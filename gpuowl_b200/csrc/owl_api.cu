@@ -98,7 +98,7 @@ struct owl_plan {
   C* F1 = nullptr;
   C* F2 = nullptr;
   void* tableMem = nullptr;
-  void* scratch = nullptr;  // shuttle, flags, ctl, roe, small outputs
+  void* scratch = nullptr;  // shuttle, ctl, roe, small outputs
   int32_t* small = nullptr; // 64 gathered words
   unsigned long long* sum = nullptr;
   int* eq = nullptr;
@@ -618,7 +618,6 @@ void sync_and_check(owl_plan* p) {
     // words together, before anything of the plan runs again
     uint32_t G = p->H / kR;
     ck(cudaMemsetAsync(p->args.ctl, 0, sizeof(owl::Ctl), p->stream), "reset ctl");
-    ck(cudaMemsetAsync(p->args.flags, 0, G * sizeof(uint32_t), p->stream), "reset flags");
     ck(cudaMemsetAsync(p->args.shuttle, 0, (size_t)G * p->W * sizeof(long long), p->stream), "reset carry words");
     ck(cudaStreamSynchronize(p->stream), "cudaStreamSynchronize");
     fail(OWL_ERR_TIMEOUT, "device-side carry wait timed out");
@@ -686,10 +685,10 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
   const std::vector<uint8_t> tc1B = W == (uint32_t)owl::kLtcW ? owl::line_tc_dft_digits() : std::vector<uint8_t>();
   const std::vector<owl::HostC> twH8 =
       owl::col_variant_ok((int)H, owl::COL_V8) ? owl::col_stage_tables(H, owl::COL_V8) : std::vector<owl::HostC>();
-  size_t nC = t.twW.size() + t.twH.size() + twH8.size() + t.rootH.size() + t.twLo.size() + t.twHi.size() +
-              twHtc.size();
-  size_t bytes = 256 * 20 + nC * sizeof(C) + (t.wt1.size() * 2 + t.wt2.size() * 2) * sizeof(double) +
-                 (t.x1.size() + t.x2.size() + t.p1masks.size()) * sizeof(uint32_t) + tcB.size() + tc1B.size();
+  const std::vector<owl::HostC> rootH = tcShape ? owl::root_table(H) : std::vector<owl::HostC>();
+  size_t nC = t.twW.size() + t.twH.size() + twH8.size() + rootH.size() + t.twLo.size() + t.twHi.size() + twHtc.size();
+  size_t bytes = 256 * 16 + nC * sizeof(C) + t.wt1.size() * 2 * sizeof(double) + t.p1masks.size() * sizeof(uint32_t) +
+                 tcB.size() + tc1B.size();
   ck(cudaMalloc(&p->tableMem, bytes), "cudaMalloc(tables)");
   std::vector<char> host(bytes, 0);
   char* hcur = host.data();
@@ -703,17 +702,13 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
   p->args.twW = reinterpret_cast<const C*>(dbase + put(t.twW.data(), t.twW.size() * sizeof(C)));
   p->twHv16 = reinterpret_cast<const C*>(dbase + put(t.twH.data(), t.twH.size() * sizeof(C)));
   if (!twH8.empty()) { p->twHv8 = reinterpret_cast<const C*>(dbase + put(twH8.data(), twH8.size() * sizeof(C))); }
-  p->args.rootH = reinterpret_cast<const C*>(dbase + put(t.rootH.data(), t.rootH.size() * sizeof(C)));
   p->args.twLo = reinterpret_cast<const C*>(dbase + put(t.twLo.data(), t.twLo.size() * sizeof(C)));
   p->args.twHi = reinterpret_cast<const C*>(dbase + put(t.twHi.data(), t.twHi.size() * sizeof(C)));
   p->args.wt1 = reinterpret_cast<const double*>(dbase + put(t.wt1.data(), t.wt1.size() * sizeof(double)));
   p->args.iwt1 = reinterpret_cast<const double*>(dbase + put(t.iwt1.data(), t.iwt1.size() * sizeof(double)));
-  p->args.x1 = reinterpret_cast<const uint32_t*>(dbase + put(t.x1.data(), t.x1.size() * sizeof(uint32_t)));
-  p->args.wt2 = reinterpret_cast<const double*>(dbase + put(t.wt2.data(), t.wt2.size() * sizeof(double)));
-  p->args.iwt2 = reinterpret_cast<const double*>(dbase + put(t.iwt2.data(), t.iwt2.size() * sizeof(double)));
-  p->args.x2 = reinterpret_cast<const uint32_t*>(dbase + put(t.x2.data(), t.x2.size() * sizeof(uint32_t)));
   p->args.p1masks = reinterpret_cast<const uint2*>(dbase + put(t.p1masks.data(), t.p1masks.size() * sizeof(uint32_t)));
   if (tcShape) {
+    p->args.rootH = reinterpret_cast<const C*>(dbase + put(rootH.data(), rootH.size() * sizeof(C)));
     p->twHtc = reinterpret_cast<const C*>(dbase + put(twHtc.data(), twHtc.size() * sizeof(C)));
     p->tcB = reinterpret_cast<const unsigned char*>(dbase + put(tcB.data(), tcB.size()));
   }
@@ -725,10 +720,10 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
   ck(cudaMalloc(&p->F1, (size_t)p->hN * sizeof(C)), "cudaMalloc(F1)");
   ck(cudaMalloc(&p->F2, (size_t)p->hN * sizeof(C)), "cudaMalloc(F2)");
 
-  // scratch: carry shuttle, flags, control word, ROE slots, small outputs
+  // scratch: carry shuttle, control word, ROE slots, small outputs
   const uint32_t G = H / kR;
   const uint32_t nw = owl::n_words(E), packBlocks = (N + owl::kPackDigits - 1) / owl::kPackDigits;
-  size_t sbytes = 256 * 14 + (size_t)G * W * sizeof(long long) + G * sizeof(uint32_t) + sizeof(owl::Ctl) +
+  size_t sbytes = 256 * 13 + (size_t)G * W * sizeof(long long) + sizeof(owl::Ctl) +
                   (size_t)(nw + 2) * sizeof(uint32_t) + packBlocks * sizeof(uint32_t) + sizeof(owl::PackCtl) +
                   2 * owl::kPendingCap * sizeof(long long) + 2 * kTsCap * sizeof(unsigned long long) +
                   kRoeCap * sizeof(float) + 64 * sizeof(int32_t) + sizeof(unsigned long long) + sizeof(int);
@@ -737,7 +732,6 @@ void plan_create(int device, uint32_t E, uint32_t W, uint32_t H, owl_plan** out)
   ck(cudaStreamSynchronize(p->stream), "cudaStreamSynchronize");
   char* cur = static_cast<char*>(p->scratch);
   p->args.shuttle = carve<long long>(cur, (size_t)G * W);
-  p->args.flags = carve<uint32_t>(cur, G);
   p->args.ctl = carve<owl::Ctl>(cur, 1);
   p->args.pending = carve<long long>(cur, 2 * owl::kPendingCap);
   p->args.tsStart = carve<unsigned long long>(cur, kTsCap);
@@ -1451,12 +1445,10 @@ int owl_probe_wait_timeout(owl_plan* plan) {
   return guarded([&] {
     check_plan(plan);
     DeviceGuard dg(plan->device);
-    // an index past the line groups' flags that nothing ever sets: the flags
-    // array is followed by the control block, so use the Ctl padding word
-    owl::Args a = plan->args;
-    a.flags = &plan->args.ctl->pad[0];
-    ck(cudaMemsetAsync(a.flags, 0, sizeof(uint32_t), plan->stream), "clear probe flag");
-    owl::k_wait_probe<<<1, 32, 0, plan->stream>>>(a, 0);
+    // a word that nothing ever sets: padding of the control block
+    uint32_t* flag = &plan->args.ctl->pad[0];
+    ck(cudaMemsetAsync(flag, 0, sizeof(uint32_t), plan->stream), "clear probe flag");
+    owl::k_wait_probe<<<1, 32, 0, plan->stream>>>(plan->args, flag);
     ck(cudaGetLastError(), "probe launch");
     sync_and_check(plan);
   });

@@ -54,7 +54,6 @@ __device__ __forceinline__ unsigned long long gtimer() {
 }
 // the carry lookback polls without sleeping: each poll is already an L2 round trip, and a
 // __nanosleep between polls measured 1.4 us slower per line pass at 8M
-__device__ __forceinline__ void spin_pause() {}
 __device__ __forceinline__ void poll_pause() {}
 
 // Programmatic dependent launch. A kernel launched with programmatic stream serialization may be

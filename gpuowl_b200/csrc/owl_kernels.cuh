@@ -37,8 +37,11 @@ enum : uint32_t { DEVERR_WAIT = 1u, DEVERR_PENDING = 2u };
 constexpr uint32_t kPendingCap = 1024;
 
 struct Args {
-  // the carry's two FP64 constants first, as a 16-byte-aligned pair (with them at offset 184 the
-  // 8M line pass spilled a register and ran 1.8 us slower)
+  // The order matters to the line pass, whose registers are full: the members' offsets decide which of them
+  // the compiler loads as 16-byte pairs. The carry's two FP64 constants come first, as such a pair (at
+  // offset 184 the 8M line pass spilled a register and ran 1.8 us slower); with tc1B behind timeoutNs
+  // instead of before ctl it spilled 72 bytes instead of 40, and an 8M iteration took 100.7 instead of
+  // 98.1 us, a 64K one 9.3 instead of 9.1.
   double scaleLo;      // 2^bitsLo
   double iscaleLo;     // 2^-bitsLo
   const C* twW;    // stage tables of the width FFT (tw_offsets(W, 16/R) layout), then the records of the
@@ -50,15 +53,11 @@ struct Args {
   const C* twHi;   // w_hN^(i << loShift)
   const double* wt1;   // per column j1: 2^(X1/N), column wl_col(t) + (W/RL) r at 2 (t + (W/RL) (r/2)) + r % 2
   const double* iwt1;  // per column j1: 2^(-X1/N), in the same order
-  const uint32_t* x1;  // per column j1: X1 = step*2H*j1 mod N
-  const double* wt2;   // per (line j2, e): 2^(X2/N)
-  const double* iwt2;  // per (line j2, e): 2^(-X2/N) / (4 hN)
-  const uint32_t* x2;  // per (line j2, e): X2 = step*(2 j2 + e) mod N
   const uint2* p1masks; // per (line group g, pass-1 thread t): the big-word and wrap bits of the thread's
                         // 32 words, bit (r R + ll) 2 + e for column wl_col(t) + (W/RL) r, line g R + ll, word e
   long long* shuttle;  // carry words, (H/R) x W in wt1's order: the carry plus an offset, above a tag bit
   long long* pending;  // (word index, carry) pairs, kPendingCap entries
-  uint32_t* flags;     // per line group
+  const unsigned char* tc1B;  // the split line pass's 16-point DFT digit planes (W = 2048), else null
   Ctl* ctl;
   float* roe;          // per-launch max round-off slots
   unsigned long long* tsStart;  // per-launch earliest CTA start (%globaltimer), profiling only
@@ -68,7 +67,6 @@ struct Args {
   uint32_t eModN;      // E % N (a word is big iff its extra < E % N)
   uint32_t loShift;
   unsigned long long timeoutNs;
-  const unsigned char* tc1B;  // the split line pass's 16-point DFT digit planes (W = 2048), else null
 };
 
 enum : int { P1_FUSED = 0, P1_IN = 1, P1_OUT = 2 };
@@ -377,15 +375,15 @@ static __global__ void k_carry_fixup_group(const __grid_constant__ GroupArgs ga)
   carry_fixup(ga.a[blockIdx.x], ga.words[blockIdx.x]);
 }
 
-// timeout probe: wait on a flag that is never set, with the pass-1 wait loop
-static __global__ void k_wait_probe(Args a, uint32_t flagIndex) {
+// timeout probe: a wait like the line pass's on a flag that is never set
+static __global__ void k_wait_probe(Args a, const uint32_t* flag) {
   if (threadIdx.x == 0) {
     unsigned long long t0 = gtimer();
     bool ok = false;
     for (uint32_t it = 0; it < (1u << 30); ++it) {
-      if (ld_acquire(a.flags + flagIndex) != 0u) { ok = true; break; }
+      if (ld_acquire(flag) != 0u) { ok = true; break; }
       if ((it & 255u) == 255u && gtimer() - t0 > a.timeoutNs) { break; }
-      spin_pause();
+      poll_pause();
     }
     if (!ok) { atomicOr(&a.ctl->error, DEVERR_WAIT); }
   }

@@ -7,7 +7,7 @@
 // allocator (cudaMalloc and cudaFree can block on the device and take an
 // unbounded time), and plug-ins whose host forbids them to allocate. For them
 // this entry point keeps every piece of scratch the squaring needs -- the FFT
-// state, the carry rows and flags, the control word, the twiddle and weight
+// state, the carry rows, the control word, the twiddle and weight
 // tables -- in one file-scope device array of a fixed size, so the library
 // never calls cudaMalloc, cudaFree or any other allocating routine on this path
 // (the tables are computed on the device).
@@ -65,7 +65,7 @@ size_t up256(size_t x) { return (x + 255) & ~size_t(255); }
 
 // byte layout of the scratch for one shape; returns the total size
 struct Layout {
-  size_t F, shuttle, pending, flags, ctl, roe, twW, twH, twLo, twHi, wt1, iwt1, x1, wt2, iwt2, x2, masks, total;
+  size_t F, shuttle, pending, ctl, roe, twW, twH, twLo, twHi, wt1, iwt1, masks, total;
 };
 Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   const uint32_t hN = W * H, G = H / kR;
@@ -78,7 +78,6 @@ Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   L.F = take((size_t)hN * sizeof(owl::C));
   L.shuttle = take((size_t)G * W * sizeof(long long));
   L.pending = take(2 * owl::kPendingCap * sizeof(long long));
-  L.flags = take(G * sizeof(uint32_t));
   L.ctl = take(sizeof(owl::Ctl));
   L.roe = take(kRoeSlots * sizeof(float));
   L.twW = take(twWn * sizeof(owl::C));
@@ -87,10 +86,6 @@ Layout layout(uint32_t W, uint32_t H, uint32_t loShift) {
   L.twHi = take((hN >> loShift) * sizeof(owl::C) + sizeof(owl::C));
   L.wt1 = take(W * sizeof(double));
   L.iwt1 = take(W * sizeof(double));
-  L.x1 = take(W * sizeof(uint32_t));
-  L.wt2 = take(2 * H * sizeof(double));
-  L.iwt2 = take(2 * H * sizeof(double));
-  L.x2 = take(2 * H * sizeof(uint32_t));
   L.masks = take((size_t)G * (kR * W / 16) * sizeof(uint2));
   L.total = o;
   return L;
@@ -160,18 +155,11 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
   }
   for (uint32_t j1 = tid; j1 < W; j1 += nth) {
     uint32_t X = (uint32_t)((step * 2 * H * (uint64_t)j1) % N);
-    const_cast<uint32_t*>(a.x1)[j1] = X;
     constexpr uint32_t RL = 16 / kR;
     const uint32_t r = j1 / (W / RL), th = (uint32_t)owl::wl_thr((int)W, (int)RL, 16, (int)(j1 % (W / RL)));
     const uint32_t at = 2 * (th + W / RL * (r / 2)) + r % 2;
     const_cast<double*>(a.wt1)[at] = exp2((double)X / N);
     const_cast<double*>(a.iwt1)[at] = exp2(-(double)X / N);
-  }
-  for (uint32_t i = tid; i < 2 * H; i += nth) {
-    uint32_t X = (uint32_t)((step * (uint64_t)i) % N);
-    const_cast<uint32_t*>(a.x2)[i] = X;
-    const_cast<double*>(a.wt2)[i] = exp2((double)X / N);
-    const_cast<double*>(a.iwt2)[i] = exp2(-(double)X / N) / (4.0 * (double)a.hN);
   }
   // pass-1 word classes (the host-side word_masks, from the same X1 / X2 formulas)
   {
@@ -196,7 +184,6 @@ __global__ void k_noalloc_tables(owl::Args a, uint32_t twWn, uint32_t twHn) {
       const_cast<uint2*>(a.p1masks)[i] = make_uint2(big, wrap);
     }
   }
-  for (uint32_t i = tid; i < H / kR; i += nth) { a.flags[i] = 0; }
   // carry words of tag 0, the tag of the launch before the first
   for (uint32_t i = tid; i < (H / kR) * W; i += nth) { a.shuttle[i] = 0; }
   if (tid == 0) {
@@ -305,14 +292,9 @@ extern "C" int owl_square_noalloc(int device, uint32_t E, uint32_t W, uint32_t H
   a.twHi = reinterpret_cast<const owl::C*>(base + L.twHi);
   a.wt1 = reinterpret_cast<const double*>(base + L.wt1);
   a.iwt1 = reinterpret_cast<const double*>(base + L.iwt1);
-  a.x1 = reinterpret_cast<const uint32_t*>(base + L.x1);
-  a.wt2 = reinterpret_cast<const double*>(base + L.wt2);
-  a.iwt2 = reinterpret_cast<const double*>(base + L.iwt2);
-  a.x2 = reinterpret_cast<const uint32_t*>(base + L.x2);
   a.p1masks = reinterpret_cast<const uint2*>(base + L.masks);
   a.shuttle = reinterpret_cast<long long*>(base + L.shuttle);
   a.pending = reinterpret_cast<long long*>(base + L.pending);
-  a.flags = reinterpret_cast<uint32_t*>(base + L.flags);
   a.ctl = reinterpret_cast<owl::Ctl*>(base + L.ctl);
   a.roe = reinterpret_cast<float*>(base + L.roe);
   a.E = E;

@@ -205,11 +205,17 @@ inline std::vector<HostC> line_tables(uint32_t W, uint32_t H, const Roots& roots
   return t;
 }
 
+// w_n^i, i < n
+inline std::vector<HostC> root_table(uint32_t n) {
+  std::vector<HostC> r(n);
+  for (uint32_t i = 0; i < n; ++i) { r[i] = root(n, i); }
+  return r;
+}
+
 struct Tables {
   uint32_t E = 0, N = 0, W = 0, H = 0, hN = 0, loShift = 0;
-  std::vector<HostC> twW, twH, rootH, twLo, twHi;
-  std::vector<double> wt1, iwt1, wt2, iwt2;
-  std::vector<uint32_t> x1, x2;
+  std::vector<HostC> twW, twH, twLo, twHi;
+  std::vector<double> wt1, iwt1;
   std::vector<uint32_t> p1masks;  // (bigmask, wrapmask) per (line group, pass-1 thread)
 };
 
@@ -310,18 +316,16 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
   const Roots roots(t.hN);
   t.loShift = roots.lo_shift();
   t.twH = col_stage_tables(H, COL_V16);
-  t.rootH.resize(H);
-  for (uint32_t i = 0; i < H; ++i) { t.rootH[i] = root(H, i); }
   t.twLo = roots.lo();
   t.twHi = roots.hi();
 
   const uint64_t step = N - (E % N);
-  t.x1.resize(W);
+  std::vector<uint32_t> x1(W), x2(2 * H);
   t.wt1.resize(W);
   t.iwt1.resize(W);
   for (uint32_t j1 = 0; j1 < W; ++j1) {
     uint32_t X = (uint32_t)((step * 2 * H * (uint64_t)j1) % N);
-    t.x1[j1] = X;
+    x1[j1] = X;
     // in the line pass's thread order
     constexpr uint32_t RL = 16 / kLinesPerBlock;
     const uint32_t r = j1 / (W / RL), th = (uint32_t)wl_thr((int)W, (int)RL, 16, (int)(j1 % (W / RL)));
@@ -329,18 +333,16 @@ inline Tables make_tables(uint32_t E, uint32_t W, uint32_t H) {
     t.wt1[at] = (double)exp2l((long double)X / N);
     t.iwt1[at] = (double)exp2l(-(long double)X / N);
   }
-  t.x2.resize(2 * H);
-  t.wt2.resize(2 * H);
-  t.iwt2.resize(2 * H);
+  std::vector<double> wt2(2 * H), iwt2(2 * H);
   const long double norm = 1.0L / (4.0L * (long double)t.hN);
   for (uint32_t i = 0; i < 2 * H; ++i) {
     uint32_t X = (uint32_t)((step * (uint64_t)i) % N);
-    t.x2[i] = X;
-    t.wt2[i] = (double)exp2l((long double)X / N);
-    t.iwt2[i] = (double)(exp2l(-(long double)X / N) * norm);
+    x2[i] = X;
+    wt2[i] = (double)exp2l((long double)X / N);
+    iwt2[i] = (double)(exp2l(-(long double)X / N) * norm);
   }
-  t.twW = line_tables(W, H, roots, t.wt2.data(), t.iwt2.data());
-  t.p1masks = word_masks(E, W, H, t.x1.data(), t.x2.data());
+  t.twW = line_tables(W, H, roots, wt2.data(), iwt2.data());
+  t.p1masks = word_masks(E, W, H, x1.data(), x2.data());
   return t;
 }
 

@@ -39,7 +39,6 @@ struct EmuPlan {
   Args a{};
   std::vector<C> twW, twH, rootH, twLo, twHi, F1, F2;
   std::vector<long long> shuttle, pending;
-  std::vector<uint32_t> flags;
   Ctl ctl{};
   std::vector<float> roe;
   int roePos = 0;
@@ -70,31 +69,23 @@ void init(EmuPlan& p, uint32_t E, uint32_t W, uint32_t H) {
     }
   }
   p.twH = toC(p.t.twH);
-  p.rootH = toC(p.t.rootH);
   p.twLo = toC(p.t.twLo);
   p.twHi = toC(p.t.twHi);
   p.F1.assign(p.t.hN, make_double2(0, 0));
   p.F2.assign(p.t.hN, make_double2(0, 0));
   p.shuttle.assign((size_t)(H / kR) * W, 0);
   p.pending.assign(2 * kPendingCap, 0);
-  p.flags.assign(H / kR, 0);
   p.roe.assign(4096, 0.0f);
   Args& a = p.a;
   a.twW = p.twW.data();
   a.twH = p.twH.data();
-  a.rootH = p.rootH.data();
   a.twLo = p.twLo.data();
   a.twHi = p.twHi.data();
   a.wt1 = p.t.wt1.data();
   a.iwt1 = p.t.iwt1.data();
-  a.x1 = p.t.x1.data();
-  a.wt2 = p.t.wt2.data();
-  a.iwt2 = p.t.iwt2.data();
-  a.x2 = p.t.x2.data();
   a.p1masks = reinterpret_cast<const uint2*>(p.t.p1masks.data());
   a.shuttle = p.shuttle.data();
   a.pending = p.pending.data();
-  a.flags = p.flags.data();
   a.ctl = &p.ctl;
   a.roe = p.roe.data();
   a.E = E;
@@ -118,6 +109,8 @@ void init(EmuPlan& p, uint32_t E, uint32_t W, uint32_t H) {
   const int spf = sp ? std::atoi(sp) : 0;  // split flags: 1 columns, 2 lines
   if ((spf & 1) && tc_height((int)H)) {
     p.split = true;
+    p.rootH = toC(root_table(H));
+    a.rootH = p.rootH.data();
     p.twHtc = toC(stage_tables(H, 8, H == 2048 ? TcCfg<2048>::R1 : TcCfg<2560>::R1));
     p.tcB = H == 2048 ? tc_dft_digits<2048>() : tc_dft_digits<2560>();
   }

@@ -170,7 +170,6 @@ namespace owl {
 inline uint32_t ld_acquire(const uint32_t* p) {
   return std::atomic_ref<uint32_t>(*const_cast<uint32_t*>(p)).load(std::memory_order_acquire);
 }
-inline void st_release(uint32_t* p, uint32_t v) { std::atomic_ref<uint32_t>(*p).store(v, std::memory_order_release); }
 inline long long ld_relaxed(const long long* p) {
   return std::atomic_ref<long long>(*const_cast<long long*>(p)).load(std::memory_order_relaxed);
 }
@@ -180,7 +179,6 @@ inline unsigned long long gtimer() {
              std::chrono::steady_clock::now().time_since_epoch())
       .count();
 }
-inline void spin_pause() { std::this_thread::yield(); }
 inline void griddep_wait() {}
 inline void griddep_launch() {}
 inline unsigned long long l2_keep_policy() { return 0; }
