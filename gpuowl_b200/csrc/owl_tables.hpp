@@ -132,12 +132,16 @@ inline std::vector<HostC> col_stage_tables(uint32_t H, int variant) {
   return r;
 }
 
-// The column variant a plan of shape W x H starts with: the fastest of the variants built for H as
-// measured on B200 by gpuowl_b200.tune --variants (time per squaring of 1,000-squaring blocks; the
-// reference's built-in tune defaults play the same part, src/TuneEntry.cpp); owl_plan_set_column_variant
-// overrides it. 8 values a thread won at 128 x 256 (10.4 against 10.7 us), 256 x 256 (10.8-10.9
-// against 11.6-11.8) and 512 x 512 (14.1 against 14.3); two CTAs per SM at 4096 x 2560 (381.3-381.6
-// against 384.0-384.8); every other measured shape keeps 16 values a thread.
+// The column variant a plan of shape W x H starts with (the reference's built-in tune defaults play the same
+// part, src/TuneEntry.cpp); owl_plan_set_column_variant overrides it, and gpuowl_b200.tune finds the quickest.
+// Measured on B200 with the present kernels, us per squaring alone / three plans in turn / four plans grouped:
+//   128 x 256: 8 values a thread 8.6-8.9 / 3.4 / 2.5, 16 values 9.6 / 3.5 / 3.3
+//   256 x 256: 8 values 10.7 / 4.2 / 3.2, 16 values 11.0 / 4.5 / 3.4
+//   1024 x 1024 (and every shape from H = 512 up): 8 values 32.1 / 24.1 / 27.5, 16 values 28.2 / 19.8 / 23.2
+//   4096 x 2560: two CTAs per SM 304 / 281 / 294, one 326 / 307 / 315
+// Three choices date from earlier kernels and are not the quickest any more: 512 x 512 (8 values 14.2 / 7.5 /
+// 7.5, 16 values 12.8 / 6.9 / 7.0), 2048 x 2560 (one CTA 139 / 133 / 141, two 130 / 124 / 130, but a product
+// 314 against 318 three in turn) and the shapes of H <= 128 (8 values 1-5 % quicker).
 inline int default_col_variant(uint32_t W, uint32_t H) {
   if ((W == 128 && H == 256) || (W == 256 && H == 256) || (W == 512 && H == 512)) { return COL_V8; }
   if (W == 4096 && H == 2560) { return COL_V16_OCC2; }
