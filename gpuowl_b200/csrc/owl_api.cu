@@ -162,6 +162,16 @@ template <int W, int M> void setp1attr() {
      "cudaFuncSetAttribute(pass1)");
   ck(cudaFuncSetAttribute(owl::k_pass1_group<W, kR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
      "cudaFuncSetAttribute(pass1 group)");
+  if constexpr (owl::bounded_threads(kR * W / 16)) {
+    ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, M, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)sm),
+       "cudaFuncSetAttribute(pass1 of few threads)");
+    if (M == owl::P1_FUSED) {
+      ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, owl::P1_FUSED, false, false, true>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
+         "cudaFuncSetAttribute(pass1 of few threads without round-off)");
+    }
+  }
   if (M == owl::P1_FUSED) {
     ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, owl::P1_FUSED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             (int)sm),
@@ -176,6 +186,10 @@ template <int H, int M, int CV> void setp2attr_v() {
   size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
   ck(cudaFuncSetAttribute(owl::k_pass2<H, kR, M, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
      "cudaFuncSetAttribute(pass2)");
+  if constexpr (V == 16 && H == 1024) {
+    ck(cudaFuncSetAttribute(owl::k_pass2<H, kR, M, V, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
+       "cudaFuncSetAttribute(pass2 of few threads)");
+  }
   if (M == owl::P2_SQUARE) {
     ck(cudaFuncSetAttribute(owl::k_pass2_group<H, kR, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
        "cudaFuncSetAttribute(pass2 group)");
@@ -254,6 +268,16 @@ template <int W> void p1launch(owl_plan* p, int mode, C* F, int32_t* words, int 
       return;
     }
   }
+  if constexpr (owl::bounded_threads(T)) {
+    if (owl::few_threads(p->hN)) {
+      auto k = (mode == owl::P1_FUSED) ? (roeSlot >= 0 ? owl::k_pass1<W, kR, owl::P1_FUSED, true, false, true>
+                                                       : owl::k_pass1<W, kR, owl::P1_FUSED, false, false, true>)
+               : (mode == owl::P1_IN)  ? owl::k_pass1<W, kR, owl::P1_IN, true, false, true>
+                                       : owl::k_pass1<W, kR, owl::P1_OUT, true, false, true>;
+      launch_pass(p, pdl, k, grid, T, sm, p->args, F, words, roeSlot, flags, ts);
+      return;
+    }
+  }
   // a fused pass with no round-off slot runs the build without the measurement
   auto k = (mode == owl::P1_FUSED) ? (roeSlot >= 0 ? owl::k_pass1<W, kR, owl::P1_FUSED>
                                                    : owl::k_pass1<W, kR, owl::P1_FUSED, false>)
@@ -267,6 +291,15 @@ template <int H, int CV> void p2launch_v(owl_plan* p, int mode, C* F, const C* F
   constexpr int T = 2 * H / V;
   size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
   dim3 grid(p->W / 2);
+  if constexpr (V == 16 && H == 1024) {
+    if (owl::few_threads(p->hN)) {
+      auto k = (mode == owl::P2_SQUARE) ? owl::k_pass2<H, kR, owl::P2_SQUARE, V, 1>
+               : (mode == owl::P2_FWD)  ? owl::k_pass2<H, kR, owl::P2_FWD, V, 1>
+                                        : owl::k_pass2<H, kR, owl::P2_MUL, V, 1>;
+      launch_pass(p, pdl, k, grid, T, sm, p->args, F, Fb, Fq, ts);
+      return;
+    }
+  }
   auto k = (mode == owl::P2_SQUARE) ? owl::k_pass2<H, kR, owl::P2_SQUARE, V, MB>
            : (mode == owl::P2_FWD)  ? owl::k_pass2<H, kR, owl::P2_FWD, V, MB>
                                     : owl::k_pass2<H, kR, owl::P2_MUL, V, MB>;

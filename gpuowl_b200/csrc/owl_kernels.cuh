@@ -241,21 +241,29 @@ __device__ __forceinline__ C one_mul(C a, C b, C c, C d, C t2) {
 // shape in one launch (blockIdx.y = plan), which a batch of exponents uses so that one launch per
 // pass and shape replaces a launch per plan.
 
-// CTAs per SM of the one-plan line pass: 16 warps at 128 registers from 64 threads a CTA (W = 512) up. Free
-// of the bound the 64- and 128-thread kernels took 240-255 registers, 8 warps an SM, which their grids
-// (256 to 1,280 CTAs) more than fill: 4M words 57.1 -> 50.2 us per iteration alone and 53.0 -> 43.8 with
-// three plans in turn, 1M 12.1 -> 9.9 with three plans (alone 17.2 -> 18.6, the one loss: its CTAs then
-// start on fewer SMs). 20 warps (102 registers) spill: 4M 46.0. The narrower kernels run a fraction of a
-// wave and keep their registers. The 128-thread columns (H = 1024) likewise: 1M x 1024 20.1 -> 19.4.
+// CTAs per SM of the one-plan line pass: 16 warps at 128 registers from 64 threads a CTA (W = 512) up, and of
+// the 128-thread columns (H = 1024). Free of the bound the 64- and 128-thread kernels take 240-255 registers,
+// 8 warps an SM. Measured unbounded / bounded, us per squaring alone and with three plans in turn:
+//   1024 x 2048 57.5 / 51.3 and 53.0 / 43.9; 512 x 1280 28.3 / 26.2 and 15.0 / 12.3; 1024 x 640 27.6 / 26.3
+//   and 17.4 / 15.4 (20 warps, 102 registers, spill: 1024 x 2048 46.0 three in turn);
+//   512 x 1024 17.6 / 19.4 and 12.3 / 10.3, 1024 x 512 16.3 / 21.3 and 11.9 / 10.4: a plan alone loses by the
+//   bound there (its CTAs start on fewer SMs), several gain more.
+// A pass of few threads in all has nothing to fill the room with and keeps its registers (few_threads):
+//   512 x 128 10.5 / 10.5 and 4.3 / 5.0; 1024 x 64 11.7 / 11.6 and 4.7 / 5.7; columns of 64 x 1024 12.7 / 15.4
+//   and 5.0 / 6.1. The line between lies at 16,384 threads, 3.5 warps an SM: 512 x 512 13.9 / 14.4 and 7.5 /
+//   7.5, 1024 x 256 13.8 / 12.8 and 7.3 / 7.0.
 constexpr int line_blocks(int T) { return T >= 512 || T < 64 ? 1 : 512 / T; }
+constexpr bool bounded_threads(int T) { return T == 64 || T == 128; }  // of a line pass
+inline bool few_threads(uint32_t hN) { return hN / 16 < 16384; }  // 16 points a thread in both passes
 
 // ROE: measure the round-off |x - rint(x)| into roe[roeSlot]. The reference measures it on a
 // sample of iterations only, with a separate kernel build (kCarryFusedROE vs kCarryFused,
 // src/Gpu.cpp:592-596); the fused line pass without it runs about 0.8 us faster at 8M.
 // SPLIT (W = 2048 only): the first inverse and last forward radix-16 stages as INT8 tensor-core
 // GEMMs (owl_line_tc.cuh), the split-precision form of the line pass.
-template <int W, int R, int MODE, bool ROE = true, bool SPLIT = false>
-__global__ void __launch_bounds__(R * W / 16, line_blocks(R * W / 16))
+// FEW: without the bound (few_threads).
+template <int W, int R, int MODE, bool ROE = true, bool SPLIT = false, bool FEW = false>
+__global__ void __launch_bounds__(R * W / 16, FEW ? 1 : line_blocks(R * W / 16))
     k_pass1(Args a, C* __restrict__ F, int32_t* __restrict__ words, int roeSlot, int flags, int tslot) {
   const uint32_t blk = blockIdx.x;
 #include "owl_pass1_body.inc"

@@ -46,3 +46,22 @@ def test_edges_vs_gmp(oracle, W, H):
         p.modMul(a, b)
         want = oracle.gmp_square(E, oracle.gmp_square(E, wa, 18), 3, ll=True)
         assert np.array_equal(p.readOut(a), oracle.gmp_mul(E, want, wb))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H", [(512, 256), (512, 512), (1024, 128), (1024, 256), (128, 1024), (256, 1024)])
+def test_register_builds_vs_gmp(oracle, W, H):
+    """Both builds of the 64- and 128-thread passes, at the sizes on either side of the line between them, with
+    and without the round-off measurement, and a product."""
+    import gpuowl_b200 as owl
+    E = exponent(W, H)
+    wa, wb = random_words(E, 41), random_words(E, 42)
+    with owl.Plan(E, W=W, H=H, column_variant=owl.COL_V16) as p:
+        a, b = p.alloc(), p.alloc()
+        p.writeIn(a, wa)
+        p.writeIn(b, wb)
+        p.squareLoop(a, a, 17, roe=False)
+        p.squareLoop(a, a, 4)
+        assert 0 < p.readROE().max() < 0.3
+        p.modMul(a, b)
+        assert np.array_equal(p.readOut(a), oracle.gmp_mul(E, oracle.gmp_square(E, wa, 21), wb))
