@@ -365,7 +365,7 @@ def bpw_scan(shapes, iters, limit=0.3, start=16.0, step=0.25, device=0, verbose=
     for (N, W, H) in shapes:
         curve, best = [], None
         bpw = start
-        while bpw <= 21.0:
+        while bpw <= BPW_CAP:
             roe = roe_at(N, W, H, bpw, iters, device)
             curve.append((bpw, roe))
             if verbose:

@@ -49,6 +49,18 @@ def test_tune_rows_with_column_variants(tmp_path):
     assert tune.tuned_variant(1 << 22, str(js)) == 0 and tune.tuned_variant(1 << 22, None) == 0
 
 
+def test_bpw_scan_stays_below_the_plans_limit(monkeypatch):
+    """A shape whose round-off never reaches the limit is scanned up to the bits per word that a plan takes."""
+    asked = []
+    monkeypatch.setattr(tune, "roe_at", lambda N, W, H, bpw, iters, device: asked.append(bpw) or 0.01)
+    from gpuowl_b200 import build
+    monkeypatch.setattr(build, "build", lambda: None)
+    N, W, H = 8192, 64, 64
+    (_, _, best, _), = tune.bpw_scan([(N, W, H)], 10, verbose=False).values()
+    assert all(tune.next_odd_exponent(N * b) / N <= 21.0 for b in asked)
+    assert best == asked[-1] == 20.75
+
+
 @pytest.mark.gpu
 def test_small_sweep_and_z_target(owl):
     rows = tune.tune(14, 14, 50, verbose=False)
