@@ -319,7 +319,7 @@ template <int H> void p2launch(owl_plan* p, int mode, C* F, const C* Fb, C* Fq, 
 }
 
 #define OWL_FOR_SIZES(X) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
-// column heights: the powers of two, and 5 * 2^k (radix-5 middle stage) for the 5 * 2^m FFT lengths
+// column heights: the powers of two, and 5 * 2^k for the 5 * 2^m FFT lengths
 #define OWL_FOR_H_SIZES(X) OWL_FOR_SIZES(X) X(640) X(1280) X(2560)
 
 void set_attrs(uint32_t W, uint32_t H) {

@@ -380,7 +380,7 @@ template <int R, int N, int NS, int PS, int VPT = 16> __device__ __forceinline__
 // Radix plan for a line of N points whose last inverse / first forward stage
 // (radix RL) is split across lines or columns: N = R1 * M1 * M2 * RL.
 // "A order" runs the stages R1, M1, M2, RL; "B order" runs RL, M2, M1, R1.
-// n = 2^a or 5 * 2^a; the factor 5 becomes the M2 stage. r1f != 0 forces the
+// n = 2^a or 5 * 2^a; the factor 5 is the M2 stage or part of a first radix of 20. r1f != 0 forces the
 // first radix (the split-precision column pass runs a 32-point first stage).
 // vmax: the largest radix (the values per thread). 2560 and 1280 points at 16 values a thread start with
 // radix 20, run by 4 of every 5 threads: one stage and exchange less than 16 x 4 x 5 x 8, and 20
@@ -493,8 +493,9 @@ struct LineTw {
 // last (B order) radix-R1 stage leaves R1 independent sub-transforms of S = N / R1 points per row,
 // sub-transform q in the shared-memory region (row, q); a warp then owns the regions of NSUB = R1 /
 // warps values of q in both rows and runs the remaining stages in them with no barrier but its own.
-// One exchange of the transform is left that needs the whole CTA. The line and column passes had two
-// barriers per exchange, 9 to 11 per launch, now 2: at 8M barriers were the line pass's top stall.
+// One exchange of the transform is left that needs the whole CTA. A column pass has 2 block barriers, one
+// for each direction, and a fused line pass 4 (two more for its ticket and its record), where two barriers
+// per exchange made 9 to 11: at 8M barriers were the line pass's top stall.
 //
 // Index maps, A order (input index i = j + S r, output index n = q + R1 (p + M n2), M = M1 M2,
 // p = p1 + M1 p2; B order is the same graph backwards):

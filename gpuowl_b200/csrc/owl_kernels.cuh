@@ -132,10 +132,10 @@ __device__ __forceinline__ void ts_end(const Args& a, int slot) {
 
 // The line pass reads and writes the state in 128-byte lines: two neighbouring columns c, both sides of
 // the pair and both lines. With lanes on consecutive k1 a request would take only one side of each pair,
-// half of every line, which costs twice the L1 wavefronts (of the passes' 16 a value's exchanges take 8
-// per stage boundary, each state access 8 instead of 4). So lane pairs work on the butterflies j and
-// S - j (S = W/R1): at step i the first takes r = i and the second r = R1 - 1 - i, the mirror column. The
-// second keeps its values conjugated: its transform is then the first's, with the same twiddles (p1_pair).
+// half of every line: 8 L1 wavefronts for a warp's 16-byte values instead of 4. So lane pairs work on the
+// butterflies j and S - j (S = W/R1): at step i the first takes r = i and the second r = R1 - 1 - i, the
+// mirror column. The second keeps its values conjugated: its transform is then the first's, with the same
+// twiddles (conj_if, Row and at() of the line pass).
 // Lines of at least 512 points, where a region of shared memory has the 3 elements to spare that keep the
 // two halves of the pairs in different banks.
 constexpr int kPairMinW = 512;

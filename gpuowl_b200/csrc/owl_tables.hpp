@@ -227,7 +227,7 @@ struct Tables {
 constexpr uint32_t kLinesPerBlock = 2;
 
 // Shapes the library supports: W a power of two in [64, 4096]; H a power of two in
-// [64, 4096], or 5 * 2^k in {640, 1280, 2560} (a radix-5 stage in the column FFT).
+// [64, 4096], or 5 * 2^k in {640, 1280, 2560}.
 inline bool h_supported(uint32_t H) {
   return (is_pow2(H) && H >= 64 && H <= 4096) || H == 640 || H == 1280 || H == 2560;
 }

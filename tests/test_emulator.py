@@ -86,8 +86,8 @@ def splitmix_words(E, seed):
 
 @pytest.mark.parametrize("E,W,H,n,seed", [
     (1300021, 64, 640, 3, 7),     # 5 * 2^14 words, radix plan 16 * 5 * 8
-    (2500009, 64, 1280, 2, 9),    # 5 * 2^15 words, radix plan 16 * 2 * 5 * 8
-    (5600027, 64, 2560, 2, 11),   # 5 * 2^16 words, radix plan 16 * 4 * 5 * 8 (the 20M column FFT)
+    (2500009, 64, 1280, 2, 9),    # 5 * 2^15 words, radix plan 20 * 8 * 8
+    (5600027, 64, 2560, 2, 11),   # 5 * 2^16 words, radix plan 20 * 16 * 8 (the 20M column FFT)
 ])
 def test_emulated_radix5_random_start(emu, oracle, E, W, H, n, seed):
     roe, got = run(emu, "square", E, W, H, n, 0, seed)
@@ -180,12 +180,13 @@ def test_emulated_grouped_line_pass(emu, oracle, E, W, H, n, flags):
 
 
 @pytest.mark.parametrize("E,W,H,n,flags", [
-    (1999993, 1024, 64, 6, 0),    # 128-thread CTAs: all carry words requested at once, then polled
-    (4500007, 2048, 64, 4, 2),    # 256-thread CTAs: carry words polled one after another, LL
+    (1999993, 1024, 64, 6, 0),    # 128-thread CTAs
+    (4500007, 2048, 64, 4, 2),    # 256-thread CTAs, LL
 ])
 def test_emulated_self_publishing_carry_words(emu, oracle, E, W, H, n, flags):
-    """The line passes from W = 1024 up publish their carry rows word by word (never-0 encoded
-    words, each consumer thread polling and clearing its own) instead of with a flag."""
+    """The line passes publish their carry rows word by word: every word carries its launch's tag, each
+    consumer thread requests its eight at once and polls those that are not there yet. Several launches, so
+    that the tag alternates."""
     ll = bool(flags & 2)
     roe, got = run(emu, "square", E, W, H, n, flags, 13)
     want = oracle.gmp_square(E, splitmix_words(E, 13), n, ll=ll)

@@ -45,7 +45,7 @@ def test_square_large_shapes_vs_gmp(owl, oracle, E, W, H):
     assert np.array_equal(got, want)
 
 
-# 5 * 2^k FFT lengths (radix-5 middle stage of the column FFT, H = 640, 1280, 2560) and the
+# 5 * 2^k FFT lengths (H = 640, 1280, 2560: a radix-5 or radix-20 stage of the column FFT) and the
 # 512-thread 4096-point instantiations, up to the 20M (5 * 2^22) and 32M lengths
 SHAPES_WIDE = [
     (1300021, 64, 640), (2500009, 64, 1280), (20000003, 1024, 640), (40000003, 1024, 1280),

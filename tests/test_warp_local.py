@@ -31,6 +31,14 @@ def test_emulated_records_hold_what_lines_read(emu, oracle, W):  # noqa: F811
     assert np.array_equal(got, oracle.gmp_square(E, random_words(E, 9), 1))
 
 
+@pytest.mark.parametrize("H", [128, 256, 1024, 2048, 4096])
+def test_emulated_column_heights(emu, oracle, H):  # noqa: F811
+    """The plain column passes that no other emulated case runs at 16 values a thread."""
+    E = exponent(64, H)
+    _, got = run(emu, "square", E, 64, H, 1, 0, 9)
+    assert np.array_equal(got, oracle.gmp_square(E, random_words(E, 9), 1))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("W,H", EDGES)
 def test_edges_vs_gmp(oracle, W, H):
