@@ -147,65 +147,50 @@ namespace {
 
 // ---- kernel dispatch on the compile-time shape --------------------------------
 
-template <int W, int M> void setp1attr() {
-  size_t sm = (size_t)kR * owl::p1_line_stride<W, kR>() * sizeof(C);
-  if constexpr (W == owl::kLtcW) {
-    const int smx = (int)sm + owl::ltc_extra_smem();
-    ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, M, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smx),
-       "cudaFuncSetAttribute(pass1 split)");
-    if (M == owl::P1_FUSED) {
-      ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, M, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smx),
-         "cudaFuncSetAttribute(pass1 split without round-off)");
-    }
-  }
-  ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-     "cudaFuncSetAttribute(pass1)");
-  ck(cudaFuncSetAttribute(owl::k_pass1_group<W, kR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-     "cudaFuncSetAttribute(pass1 group)");
-  if constexpr (owl::bounded_threads(kR * W / 16)) {
-    ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, M, true, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)sm),
-       "cudaFuncSetAttribute(pass1 of few threads)");
-    if (M == owl::P1_FUSED) {
-      ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, owl::P1_FUSED, false, false, true>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-         "cudaFuncSetAttribute(pass1 of few threads without round-off)");
-    }
-  }
-  if (M == owl::P1_FUSED) {
-    ck(cudaFuncSetAttribute(owl::k_pass1<W, kR, owl::P1_FUSED, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)sm),
-       "cudaFuncSetAttribute(pass1 without round-off)");
-    ck(cudaFuncSetAttribute(owl::k_pass1_group<W, kR, owl::P1_FUSED, false>,
-                            cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-       "cudaFuncSetAttribute(pass1 group without round-off)");
-  }
+// the largest dynamic shared memory of the builds that a plan of hN points runs (a build's first use loads it)
+void smem_attr(const void* kernel, size_t bytes) {
+  ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "cudaFuncSetAttribute");
 }
-template <int H, int M, int CV> void setp2attr_v() {
+template <int W, int M, bool FEW> void setp1attr_b(size_t sm) {
+  smem_attr((const void*)owl::k_pass1<W, kR, M, true, false, FEW>, sm);
+  if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1<W, kR, owl::P1_FUSED, false, false, FEW>, sm); }
+}
+template <int W, int M> void setp1attr(uint32_t hN) {
+  const size_t sm = (size_t)kR * owl::p1_line_stride<W, kR>() * sizeof(C);
+  if constexpr (W == owl::kLtcW) {
+    const size_t smx = sm + owl::ltc_extra_smem();
+    smem_attr((const void*)owl::k_pass1<W, kR, M, true, true>, smx);
+    if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1<W, kR, owl::P1_FUSED, false, true>, smx); }
+  }
+  bool few = false;
+  if constexpr (owl::bounded_threads(kR * W / 16)) {
+    few = owl::few_threads(hN);
+    if (few) { setp1attr_b<W, M, true>(sm); }
+  }
+  if (!few) { setp1attr_b<W, M, false>(sm); }
+  smem_attr((const void*)owl::k_pass1_group<W, kR, M>, sm);
+  if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1_group<W, kR, owl::P1_FUSED, false>, sm); }
+}
+template <int H, int M, int CV> void setp2attr_v(uint32_t hN) {
   constexpr int V = owl::col_vpt(CV), MB = owl::col_minb(CV);
-  size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
-  ck(cudaFuncSetAttribute(owl::k_pass2<H, kR, M, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-     "cudaFuncSetAttribute(pass2)");
+  const size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
+  bool few = false;
   if constexpr (V == 16 && H == 1024) {
-    ck(cudaFuncSetAttribute(owl::k_pass2<H, kR, M, V, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-       "cudaFuncSetAttribute(pass2 of few threads)");
+    few = owl::few_threads(hN);
+    if (few) { smem_attr((const void*)owl::k_pass2<H, kR, M, V, 1>, sm); }
   }
-  if (M == owl::P2_SQUARE) {
-    ck(cudaFuncSetAttribute(owl::k_pass2_group<H, kR, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm),
-       "cudaFuncSetAttribute(pass2 group)");
-  }
+  if (!few) { smem_attr((const void*)owl::k_pass2<H, kR, M, V, MB>, sm); }
+  if (M == owl::P2_SQUARE) { smem_attr((const void*)owl::k_pass2_group<H, kR, V, MB>, sm); }
 }
 // every column variant built for H
-template <int H, int M> void setp2attr() {
-  setp2attr_v<H, M, owl::COL_V16>();
-  if constexpr (owl::col_variant_ok(H, owl::COL_V8)) { setp2attr_v<H, M, owl::COL_V8>(); }
-  if constexpr (owl::col_variant_ok(H, owl::COL_V16_OCC2)) { setp2attr_v<H, M, owl::COL_V16_OCC2>(); }
+template <int H, int M> void setp2attr(uint32_t hN) {
+  setp2attr_v<H, M, owl::COL_V16>(hN);
+  if constexpr (owl::col_variant_ok(H, owl::COL_V8)) { setp2attr_v<H, M, owl::COL_V8>(hN); }
+  if constexpr (owl::col_variant_ok(H, owl::COL_V16_OCC2)) { setp2attr_v<H, M, owl::COL_V16_OCC2>(hN); }
 }
 
 template <int H, int M> void setp2tcattr() {
-  ck(cudaFuncSetAttribute(owl::k_pass2_tc<H, kR, M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                          owl::TcCfg<H>::SMEM),
-     "cudaFuncSetAttribute(pass2 split)");
+  smem_attr((const void*)owl::k_pass2_tc<H, kR, M>, owl::TcCfg<H>::SMEM);
 }
 
 // Launches a pass kernel on the plan's stream. With `pdl` it is a programmatic dependent of the
@@ -326,9 +311,9 @@ void set_attrs(uint32_t W, uint32_t H) {
   switch (W) {
 #define CASE_W(n)                  \
   case n:                          \
-    setp1attr<n, owl::P1_FUSED>(); \
-    setp1attr<n, owl::P1_IN>();    \
-    setp1attr<n, owl::P1_OUT>();   \
+    setp1attr<n, owl::P1_FUSED>(W * H); \
+    setp1attr<n, owl::P1_IN>(W * H);    \
+    setp1attr<n, owl::P1_OUT>(W * H);   \
     break;
     OWL_FOR_SIZES(CASE_W)
 #undef CASE_W
@@ -338,9 +323,9 @@ void set_attrs(uint32_t W, uint32_t H) {
   switch (H) {
 #define CASE_H(n)                   \
   case n:                           \
-    setp2attr<n, owl::P2_SQUARE>(); \
-    setp2attr<n, owl::P2_FWD>();    \
-    setp2attr<n, owl::P2_MUL>();    \
+    setp2attr<n, owl::P2_SQUARE>(W * H); \
+    setp2attr<n, owl::P2_FWD>(W * H);    \
+    setp2attr<n, owl::P2_MUL>(W * H);    \
     break;
     OWL_FOR_H_SIZES(CASE_H)
 #undef CASE_H

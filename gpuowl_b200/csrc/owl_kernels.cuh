@@ -37,11 +37,12 @@ enum : uint32_t { DEVERR_WAIT = 1u, DEVERR_PENDING = 2u };
 constexpr uint32_t kPendingCap = 1024;
 
 struct Args {
-  // The order matters to the line pass, whose registers are full: the members' offsets decide which of them
-  // the compiler loads as 16-byte pairs. The carry's two FP64 constants come first, as such a pair (at
-  // offset 184 the 8M line pass spilled a register and ran 1.8 us slower); with tc1B behind timeoutNs
-  // instead of before ctl it spilled 72 bytes instead of 40, and an 8M iteration took 100.7 instead of
-  // 98.1 us, a 64K one 9.3 instead of 9.1.
+  // The offsets matter: the passes' registers are full, and the members' places decide which of them the
+  // compiler loads as pairs. The carry's two FP64 constants come first, as a 16-byte-aligned pair (at offset
+  // 184 the 8M line pass spilled a register and ran 1.8 us slower), and the two gaps keep the others where
+  // they were measured: without them an 8M iteration took 100.7 instead of 98.1 us and a 64K one 9.3 instead
+  // of 9.1; with tc1B in front of ctl instead, 1M (three plans in turn) 10.7 instead of 10.5 and the split
+  // form at 8M 168 instead of 166.
   double scaleLo;      // 2^bitsLo
   double iscaleLo;     // 2^-bitsLo
   const C* twW;    // stage tables of the width FFT (tw_offsets(W, 16/R) layout), then the records of the
@@ -53,11 +54,12 @@ struct Args {
   const C* twHi;   // w_hN^(i << loShift)
   const double* wt1;   // per column j1: 2^(X1/N), column wl_col(t) + (W/RL) r at 2 (t + (W/RL) (r/2)) + r % 2
   const double* iwt1;  // per column j1: 2^(-X1/N), in the same order
+  const void* gap0[4];
   const uint2* p1masks; // per (line group g, pass-1 thread t): the big-word and wrap bits of the thread's
                         // 32 words, bit (r R + ll) 2 + e for column wl_col(t) + (W/RL) r, line g R + ll, word e
   long long* shuttle;  // carry words, (H/R) x W in wt1's order: the carry plus an offset, above a tag bit
   long long* pending;  // (word index, carry) pairs, kPendingCap entries
-  const unsigned char* tc1B;  // the split line pass's 16-point DFT digit planes (W = 2048), else null
+  const void* gap1;
   Ctl* ctl;
   float* roe;          // per-launch max round-off slots
   unsigned long long* tsStart;  // per-launch earliest CTA start (%globaltimer), profiling only
@@ -67,6 +69,7 @@ struct Args {
   uint32_t eModN;      // E % N (a word is big iff its extra < E % N)
   uint32_t loShift;
   unsigned long long timeoutNs;
+  const unsigned char* tc1B;  // the split line pass's 16-point DFT digit planes (W = 2048), else null
 };
 
 enum : int { P1_FUSED = 0, P1_IN = 1, P1_OUT = 2 };
