@@ -151,9 +151,12 @@ namespace {
 void smem_attr(const void* kernel, size_t bytes) {
   ck(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes), "cudaFuncSetAttribute");
 }
-template <int W, int M, bool FEW> void setp1attr_b(size_t sm) {
-  smem_attr((const void*)owl::k_pass1<W, kR, M, true, false, FEW>, sm);
-  if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1<W, kR, owl::P1_FUSED, false, false, FEW>, sm); }
+// the fused line pass without the round-off measurement
+template <int W> auto line_no_roe(uint32_t hN) {
+  if constexpr (owl::bounded_lines(kR * W / 16)) {
+    if (owl::few_line_threads(hN)) { return owl::k_pass1<W, kR, owl::P1_FUSED, false, false, true>; }
+  }
+  return owl::k_pass1<W, kR, owl::P1_FUSED, false>;
 }
 template <int W, int M> void setp1attr(uint32_t hN) {
   const size_t sm = (size_t)kR * owl::p1_line_stride<W, kR>() * sizeof(C);
@@ -162,21 +165,19 @@ template <int W, int M> void setp1attr(uint32_t hN) {
     smem_attr((const void*)owl::k_pass1<W, kR, M, true, true>, smx);
     if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1<W, kR, owl::P1_FUSED, false, true>, smx); }
   }
-  bool few = false;
-  if constexpr (owl::bounded_threads(kR * W / 16)) {
-    few = owl::few_threads(hN);
-    if (few) { setp1attr_b<W, M, true>(sm); }
-  }
-  if (!few) { setp1attr_b<W, M, false>(sm); }
+  smem_attr((const void*)owl::k_pass1<W, kR, M>, sm);
   smem_attr((const void*)owl::k_pass1_group<W, kR, M>, sm);
-  if (M == owl::P1_FUSED) { smem_attr((const void*)owl::k_pass1_group<W, kR, owl::P1_FUSED, false>, sm); }
+  if constexpr (M == owl::P1_FUSED) {
+    smem_attr((const void*)line_no_roe<W>(hN), sm);
+    smem_attr((const void*)owl::k_pass1_group<W, kR, M, false>, sm);
+  }
 }
 template <int H, int M, int CV> void setp2attr_v(uint32_t hN) {
   constexpr int V = owl::col_vpt(CV), MB = owl::col_minb(CV);
   const size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
   bool few = false;
   if constexpr (V == 16 && H == 1024) {
-    few = owl::few_threads(hN);
+    few = owl::few_column_threads(hN);
     if (few) { smem_attr((const void*)owl::k_pass2<H, kR, M, V, 1>, sm); }
   }
   if (!few) { smem_attr((const void*)owl::k_pass2<H, kR, M, V, MB>, sm); }
@@ -253,19 +254,8 @@ template <int W> void p1launch(owl_plan* p, int mode, C* F, int32_t* words, int 
       return;
     }
   }
-  if constexpr (owl::bounded_threads(T)) {
-    if (owl::few_threads(p->hN)) {
-      auto k = (mode == owl::P1_FUSED) ? (roeSlot >= 0 ? owl::k_pass1<W, kR, owl::P1_FUSED, true, false, true>
-                                                       : owl::k_pass1<W, kR, owl::P1_FUSED, false, false, true>)
-               : (mode == owl::P1_IN)  ? owl::k_pass1<W, kR, owl::P1_IN, true, false, true>
-                                       : owl::k_pass1<W, kR, owl::P1_OUT, true, false, true>;
-      launch_pass(p, pdl, k, grid, T, sm, p->args, F, words, roeSlot, flags, ts);
-      return;
-    }
-  }
   // a fused pass with no round-off slot runs the build without the measurement
-  auto k = (mode == owl::P1_FUSED) ? (roeSlot >= 0 ? owl::k_pass1<W, kR, owl::P1_FUSED>
-                                                   : owl::k_pass1<W, kR, owl::P1_FUSED, false>)
+  auto k = (mode == owl::P1_FUSED) ? (roeSlot >= 0 ? owl::k_pass1<W, kR, owl::P1_FUSED> : line_no_roe<W>(p->hN))
            : (mode == owl::P1_IN)  ? owl::k_pass1<W, kR, owl::P1_IN>
                                    : owl::k_pass1<W, kR, owl::P1_OUT>;
   launch_pass(p, pdl, k, grid, T, sm, p->args, F, words, roeSlot, flags, ts);
@@ -277,7 +267,7 @@ template <int H, int CV> void p2launch_v(owl_plan* p, int mode, C* F, const C* F
   size_t sm = 2 * (size_t)owl::p2_col_stride<H, V>() * sizeof(C);
   dim3 grid(p->W / 2);
   if constexpr (V == 16 && H == 1024) {
-    if (owl::few_threads(p->hN)) {
+    if (owl::few_column_threads(p->hN)) {
       auto k = (mode == owl::P2_SQUARE) ? owl::k_pass2<H, kR, owl::P2_SQUARE, V, 1>
                : (mode == owl::P2_FWD)  ? owl::k_pass2<H, kR, owl::P2_FWD, V, 1>
                                         : owl::k_pass2<H, kR, owl::P2_MUL, V, 1>;

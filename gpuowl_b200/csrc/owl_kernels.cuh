@@ -251,20 +251,23 @@ __device__ __forceinline__ C one_mul(C a, C b, C c, C d, C t2) {
 //   and 17.4 / 15.4 (20 warps, 102 registers, spill: 1024 x 2048 46.0 three in turn);
 //   512 x 1024 17.6 / 19.4 and 12.3 / 10.3, 1024 x 512 16.3 / 21.3 and 11.9 / 10.4: a plan alone loses by the
 //   bound there (its CTAs start on fewer SMs), several gain more.
-// A pass of few threads in all has nothing to fill the room with and keeps its registers (few_threads):
-//   512 x 128 10.5 / 10.5 and 4.3 / 5.0; 1024 x 64 11.7 / 11.6 and 4.7 / 5.7; columns of 64 x 1024 12.7 / 15.4
-//   and 5.0 / 6.1. The line between lies at 16,384 threads, 3.5 warps an SM: 512 x 512 13.9 / 14.4 and 7.5 /
-//   7.5, 1024 x 256 13.8 / 12.8 and 7.3 / 7.0.
+// A pass of few threads in all has nothing to fill the room with and keeps its registers:
+//   columns below 16,384 threads: 64 x 1024 12.9 / 16.1 and 5.0 / 6.1, 128 x 1024 12.9 / 19.3 and 5.5 / 6.3
+//   (256 x 1024 14.7 / 14.8 and 7.0 / 7.8, where several plans fill the chip);
+//   lines below 8,192 threads without the round-off measurement: 512 x 64 10.1 / 10.4 and 3.7 / 4.6, 512 x 128
+//   9.9 / 10.3 and 4.2 / 5.0, 1024 x 64 11.5 / 11.4 and 4.6 / 5.6. At 8,192 and up a plan alone loses more (1024 x
+//   128 12.0 / 11.7, 5.1 / 5.9), and with the measurement at every size (1024 x 64 11.8 / 11.5, 4.8 / 5.8).
 constexpr int line_blocks(int T) { return T >= 512 || T < 64 ? 1 : 512 / T; }
-constexpr bool bounded_threads(int T) { return T == 64 || T == 128; }  // of a line pass
-inline bool few_threads(uint32_t hN) { return hN / 16 < 16384; }  // 16 points a thread in both passes
+constexpr bool bounded_lines(int T) { return T == 64 || T == 128; }
+inline bool few_line_threads(uint32_t hN) { return hN / 16 < 8192; }     // 16 points a thread
+inline bool few_column_threads(uint32_t hN) { return hN / 16 < 16384; }  // H = 1024 at 16 values a thread
 
 // ROE: measure the round-off |x - rint(x)| into roe[roeSlot]. The reference measures it on a
 // sample of iterations only, with a separate kernel build (kCarryFusedROE vs kCarryFused,
 // src/Gpu.cpp:592-596); the fused line pass without it runs about 0.8 us faster at 8M.
 // SPLIT (W = 2048 only): the first inverse and last forward radix-16 stages as INT8 tensor-core
 // GEMMs (owl_line_tc.cuh), the split-precision form of the line pass.
-// FEW: without the bound (few_threads).
+// FEW: without the bound (few_line_threads).
 template <int W, int R, int MODE, bool ROE = true, bool SPLIT = false, bool FEW = false>
 __global__ void __launch_bounds__(R * W / 16, FEW ? 1 : line_blocks(R * W / 16))
     k_pass1(Args a, C* __restrict__ F, int32_t* __restrict__ words, int roeSlot, int flags, int tslot) {

@@ -94,6 +94,10 @@ int main(int argc, char** argv) {
   } else if (what == "power" && argc == 5) {
     owl_plan* p = plan((uint32_t)std::atoi(argv[2]), (uint32_t)std::atoi(argv[3]), (uint32_t)std::atoi(argv[4]));
     int32_t *a = buf(p), *b = buf(p);
+    mark("square");
+    must(owl_square(p, b, a, 3, 0));
+    mark("square without round-off");
+    must(owl_square(p, b, a, 3, OWL_SQ_NO_ROE));
     mark("power");
     must(owl_exp_mul(p, a, 0xb5, b));
     for (int i = 0; i < 2; ++i) {

@@ -105,16 +105,19 @@ def test_batch_graph_follows_the_plans_settings(host_log):
 
 
 @pytest.mark.parametrize("W,H,line_few,column_few", [
-    (256, 64, False, False), (512, 64, True, False), (512, 256, True, False), (512, 512, False, False),
-    (1024, 128, True, False), (1024, 256, False, False), (64, 1024, False, True), (128, 1024, False, True),
+    (256, 64, False, False), (512, 64, True, False), (512, 128, True, False), (512, 256, False, False),
+    (1024, 64, True, False), (1024, 128, False, False), (64, 1024, False, True), (128, 1024, False, True),
     (256, 1024, False, False), (2048, 64, False, False)])
 def test_passes_of_few_threads_run_the_unbounded_builds(host_log, W, H, line_few, column_few):
-    """Line passes of 64 and 128 threads and 1024-point columns are bounded to 128 registers from 16,384
-    threads a pass up, for every mode."""
+    """Line passes of 64 and 128 threads and 1024-point columns are bounded to 128 registers, but for the fused
+    line pass without the round-off measurement below 8,192 threads and columns below 16,384."""
     log = host_log("power", W, H, 0)
-    k = [x.split()[1] for x in log["power"] + log["product"] if x.startswith("launch k_pass")]
-    lines = {x for x in k if x.startswith("k_pass1<")}
-    columns = {x for x in k if x.startswith("k_pass2<")}
-    assert len(lines) == 3 and len(columns) == 3  # fused, in, out; square, forward, multiply
-    assert {x.rstrip(">").split(",")[5] == "true" for x in lines} == {line_few}, lines
-    assert {x.rstrip(">").split(",")[4] == "1" for x in columns} == {column_few}, columns
+    few = set()
+    for section in ("square", "square without round-off", "power", "product"):
+        k = [x.split()[1].rstrip(">") for x in log[section] if x.startswith("launch k_pass")]
+        lines = {x for x in k if x.startswith("k_pass1<")}
+        columns = {x for x in k if x.startswith("k_pass2<")}
+        assert lines and columns
+        few |= {x.split("<")[1].split(",", 2)[2] for x in lines if x.endswith(",true") and x.count(",") == 5}
+        assert {x.split(",")[4] == "1" for x in columns} == {column_few}, columns
+    assert few == ({"0,false,false,true"} if line_few else set())
